@@ -409,7 +409,7 @@ int clear_flags(cr_ctx* ctx) {
   s.bar_count = 0;
   s.stalled = 0;
   s.pbar = 0;
-  s.pflag[0] = s.pflag[1] = s.pflag[2] = 0;
+  s.pflag[0] = 0;
   s.pbase = 0;
   *ctx->status_h = s;
   CR_TRY(cudaMemcpyAsync(ctx->status, ctx->status_h, sizeof(DevStatus), cudaMemcpyHostToDevice, ctx->stream));
@@ -761,7 +761,7 @@ int rerun_degraded(cr_ctx* ctx, int b0, const DevStatus& start, int kind, long n
   DevStatus s = start;
   s.abort = s.overflow = s.rebuild = s.converged = s.nonfinite = s.stalled = 0;
   s.done_ctr = s.bar_count = s.pbar = 0;
-  s.pflag[0] = s.pflag[1] = s.pflag[2] = 0;
+  s.pflag[0] = 0;
   s.pbase = s.steps_left = 0;
   *ctx->status_h = s;
   if ((rc = upload(ctx, ctx->status, ctx->status_h, sizeof(DevStatus)))) return rc;

@@ -7,10 +7,10 @@ namespace cr {
 
 template <int POT, int INTER, int MODE>
 static void launch_tile_t(const LaunchCfg& c, const SysParams& p, const SysArrays& a, const StepArgs& s) {
-  if (c.lanes == 1) launch_k(c.pdl, k_tile<POT, INTER, MODE, 128, 1, PREC_FP64>, dim3(c.grid), dim3(128), c.stream, p, a, s);
-  else if (c.lanes == 4) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 4, PREC_FP64>, dim3(c.grid), dim3(256), c.stream, p, a, s);
-  else if (c.lanes == 8) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 8, PREC_FP64>, dim3(c.grid), dim3(256), c.stream, p, a, s);
-  else launch_k(c.pdl, k_tile<POT, INTER, MODE, 192, 2, PREC_FP64>, dim3(c.grid), dim3(192), c.stream, p, a, s);
+  if (c.lanes == 1) launch_k(c.pdl, k_tile<POT, INTER, MODE, 128, 1, PREC_FP64>, dim3(c.grid), dim3(128), c.stream, 0, p, a, s);
+  else if (c.lanes == 4) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 4, PREC_FP64>, dim3(c.grid), dim3(256), c.stream, 0, p, a, s);
+  else if (c.lanes == 8) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 8, PREC_FP64>, dim3(c.grid), dim3(256), c.stream, 0, p, a, s);
+  else launch_k(c.pdl, k_tile<POT, INTER, MODE, 192, 2, PREC_FP64>, dim3(c.grid), dim3(192), c.stream, 0, p, a, s);
 }
 
 void launch_tile(const LaunchCfg& c, int pot, int inter, int mode, const SysParams& p_in, const SysArrays& a,
@@ -70,13 +70,18 @@ static TileStepsFn steps_fn(int pot, int inter, int lanes, int precision) {
   return precision == CR_PRECISION_MIXED ? tile_steps_fn_mixed(pot, inter, lanes) : tile_steps_fn_fp64(pot, inter, lanes);
 }
 
+// the staged neighbourhood (cr_tile_kernel.cuh)
+static size_t steps_smem(int lanes) { return lanes == 1 ? stage_bytes<128>() : stage_bytes<96>(); }
+
 int tile_steps_max_blocks(int pot, int inter, int lanes, int precision) {
   TileStepsFn k = steps_fn(pot, inter, lanes, precision);
   if (!k) return 0;
   int dev = 0, sms = 0, occ = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, lanes == 1 ? 128 : 192, 0) != cudaSuccess) return 0;
+  const size_t smem = steps_smem(lanes);
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, lanes == 1 ? 128 : 192, smem) != cudaSuccess) return 0;
   return occ * sms;
 }
 
@@ -85,7 +90,7 @@ cudaError_t launch_tile_steps(const LaunchCfg& c, int pot, int inter, const SysP
   TileStepsFn k = steps_fn(pot, inter, c.lanes, c.precision);
   if (!k) return cudaErrorInvalidValue;
   const SysParams p = with_f32_constants(p_in);
-  return launch_k(c.pdl, k, dim3(c.grid), dim3(c.lanes == 1 ? 128 : 192), c.stream, p, a, s);
+  return launch_k(c.pdl, k, dim3(c.grid), dim3(c.lanes == 1 ? 128 : 192), c.stream, steps_smem(c.lanes), p, a, s);
 }
 
 }  // namespace cr

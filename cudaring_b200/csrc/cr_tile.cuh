@@ -305,7 +305,7 @@ __device__ __forceinline__ float sign_of_f(float c) {
 // add the unit energy, which the reference books on the rings of t and of o.
 //
 // Inputs are offsets from t: tq = t - q (minimum image), w = t - o, and the
-// segment vectors seg = o - q, pseg = q - qq; tabs, qabs are t and q in box
+// segment vectors seg = o - q, pseg = q - qq, inv_len = 1 / |seg|; tabs, qabs are t and q in box
 // coordinates.  The reference forms t - qq and the projection point
 // q + proj * seg explicitly.  Here
 //   * FP64 forms the projection point as the reference does, in box
@@ -340,10 +340,9 @@ __device__ __forceinline__ bool pair_eval_t(const SysParams& p, float d2, float 
 }
 
 template <int POT, bool ROLE1, typename T, class B, typename T2 = typename Vec2<T>::type>
-__device__ __forceinline__ void smooth_core(const SysParams& p, const B& bx, T2 tq, T tq2, T2 w, T2 seg, T len2,
+__device__ __forceinline__ void smooth_core(const SysParams& p, const B& bx, T2 tq, T tq2, T2 w, T2 seg, T inv_len,
                                             T2 pseg, T rsum, T inv_rsum, double2 tabs, double2 qabs, T2& ft,
                                             T2& fo, T2& fq, double& e) {
-  const T inv_len = rsq(len2);
   const T inv_lsq = inv_len * inv_len;
   const T proj = (tq.x * seg.x + tq.y * seg.y) * inv_lsq;
   const T pc = tq.x * pseg.x + tq.y * pseg.y;

@@ -37,11 +37,17 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   const int4 tile = a.tiles[blockIdx.x];
   bool stalled = false;
   int rebuild = 0;
+  extern __shared__ __align__(16) unsigned char s_stage[];
+  Stage<BLOCK / L> g(s_stage);
   const int n = nmax > 0 ? nmax : pending;
+  if (n > 0) {
+    const BatchSys& bs = s.bsys[tile.x];
+    stage_build<INTER, BLOCK, L>(p, bs.box, a, tile, s.last_pos, bs.disp_cutoff, pot_range_f<POT>(p), g);
+  }
   for (int j = 0; j < n; j++) {
     if (!(j == 0 && pending)) {
       for (int v = tile.z + threadIdx.x; v < tile.w; v += BLOCK) bfire_prekick(f, v);
-      if (!steps_barrier(st)) {
+      if (steps_barrier(st) < 0) {
         stalled = true;
         break;
       }
@@ -54,8 +60,8 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
         break;
       }
     }
-    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, true, 2>(p, a, s, a.pos, s.pos_out, 0ull, nullptr);
-    if (!steps_barrier(st)) {
+    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, true, 2>(p, a, s, a.pos, s.pos_out, 0ull, nullptr, false, &g, tile);
+    if (steps_barrier(st) < 0) {
       stalled = true;
       break;
     }
@@ -73,6 +79,9 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
 }
 
 namespace {
+
+// dynamic shared memory of the two shapes (tiles of 128 and 96 vertices)
+size_t stage_smem(int block) { return block == 128 ? stage_bytes<128>() : stage_bytes<96>(); }
 
 template <int POT, int INTER>
 BFireStepsFn fn_shape(int lanes, int block) {
@@ -101,13 +110,14 @@ int bfire_steps_max_blocks(BFireStepsFn fn, int block) {
   int dev = 0, sms = 0, occ = 0;
   if (!fn || cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, 0) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem(block)) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, stage_smem(block)) != cudaSuccess) return 0;
   return occ * sms;
 }
 
 void launch_bfire_steps(BFireStepsFn fn, const LaunchCfg& c, int block, const SysParams& p, const SysArrays& a,
                         const StepArgs& s, const BFire& f, int nmax) {
-  fn<<<c.grid, block, 0, c.stream>>>(p, a, s, f, nmax);
+  fn<<<c.grid, block, stage_smem(block), c.stream>>>(p, a, s, f, nmax);
 }
 
 }  // namespace cr

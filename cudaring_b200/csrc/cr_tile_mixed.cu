@@ -8,10 +8,10 @@ namespace cr {
 
 template <int POT, int INTER, int MODE>
 static void launch_mixed_t(const LaunchCfg& c, const SysParams& p, const SysArrays& a, const StepArgs& s) {
-  if (c.lanes == 1) launch_k(c.pdl, k_tile<POT, INTER, MODE, 128, 1, PREC_MIXED>, dim3(c.grid), dim3(128), c.stream, p, a, s);
-  else if (c.lanes == 4) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 4, PREC_MIXED>, dim3(c.grid), dim3(256), c.stream, p, a, s);
-  else if (c.lanes == 8) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 8, PREC_MIXED>, dim3(c.grid), dim3(256), c.stream, p, a, s);
-  else launch_k(c.pdl, k_tile<POT, INTER, MODE, 192, 2, PREC_MIXED>, dim3(c.grid), dim3(192), c.stream, p, a, s);
+  if (c.lanes == 1) launch_k(c.pdl, k_tile<POT, INTER, MODE, 128, 1, PREC_MIXED>, dim3(c.grid), dim3(128), c.stream, 0, p, a, s);
+  else if (c.lanes == 4) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 4, PREC_MIXED>, dim3(c.grid), dim3(256), c.stream, 0, p, a, s);
+  else if (c.lanes == 8) launch_k(c.pdl, k_tile<POT, INTER, MODE, 256, 8, PREC_MIXED>, dim3(c.grid), dim3(256), c.stream, 0, p, a, s);
+  else launch_k(c.pdl, k_tile<POT, INTER, MODE, 192, 2, PREC_MIXED>, dim3(c.grid), dim3(192), c.stream, 0, p, a, s);
 }
 
 void launch_tile_mixed(const LaunchCfg& c, int pot, int inter, int mode, const SysParams& p, const SysArrays& a,
