@@ -676,9 +676,9 @@ int launch_chunk(cr_ctx* ctx, const std::vector<Op>& ops, int kind, long n) {
 // NVE, Langevin and BAOAB runs of deformable rings: the drift op, then the
 // middle steps in k_tile_steps launches (each runs until its step budget, a
 // due rebuild or the end of the sequence; the one-launch build follows
-// every launch), then the final op.  Graphs of up to kStepsLaunches such
-// pairs (sized to the steps left, one spare launch for a rebuild) are
-// launched until the device counter of middle steps reaches zero; the step
+// every launch), then the final op.  Up to kStepsLaunches such pairs (sized to
+// the steps left, one spare launch for a rebuild) go out between two reads of
+// the device counter of middle steps, until it reaches zero; the step
 // arithmetic is the per-op path's, so FP64 results are identical to it.
 constexpr int kStepsPerLaunch = 64;
 constexpr int kStepsLaunches = 16;
@@ -692,7 +692,12 @@ bool steps_eligible(cr_ctx* ctx, int kind, long nsteps) {
   return maxb >= (int)ctx->tiles_h.size();
 }
 
-int capture_steps_graph(cr_ctx* ctx, int kind, int b, int launches, GraphEntry& ge) {
+// `launches` multi-step launches, each with the build that may follow it.
+// They go to the stream one by one: a launch runs up to 64 steps, hundreds of
+// microseconds, so the host is ahead of it anyway, while a graph of them had
+// to be captured, instantiated and destroyed again for every sequence whose
+// parameters had changed (0.3 to 0.5 ms of a 200-step call).
+int launch_steps(cr_ctx* ctx, int kind, int b, int launches) {
   StepArgs s = base_args(ctx);
   s.kind = kind;
   s.pos_out = ctx->pos[b ^ 1];
@@ -707,22 +712,12 @@ int capture_steps_graph(cr_ctx* ctx, int kind, int b, int launches, GraphEntry& 
   NbrArgs nb = nbr_args(ctx, b, ctx->cut_distance);
   nb.count_update = 1;
   const int fb = nbr_fused_blocks(ctx->nv, ctx->fused_max);
-  CR_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = cudaSuccess;
-  for (int r = 0; r < launches && e == cudaSuccess; r++) {
-    e = launch_tile_steps(c, ctx->potential, inter_kind(ctx), ctx->p, a, s);
+  for (int r = 0; r < launches; r++) {
+    CR_TRY(launch_tile_steps(c, ctx->potential, inter_kind(ctx), ctx->p, a, s));
     launch_nbr_fused(ctx->stream, ctx->p, ctx->grid, nb, fb, 0, true);
+    ctx->launches += 2;
   }
-  cudaGraph_t out = nullptr;
-  const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &out);
-  if (e == cudaSuccess) e = e2;
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&ge.exec, out, 0);
-  if (e != cudaSuccess) {
-    if (out) cudaGraphDestroy(out);
-    return ctx->fail(CR_ECUDA, std::string("multi-step graph: ") + cudaGetErrorString(e));
-  }
-  ge.graph = out;
-  ge.launches = 2 * launches;
+  CR_TRY(cudaGetLastError());
   return CR_OK;
 }
 
@@ -792,15 +787,7 @@ int run_steps(cr_ctx* ctx, int kind, long nsteps) {
   for (;;) {
     const int launches =
         (int)std::min<long long>(kStepsLaunches, std::max<long long>(2, (left + kStepsPerLaunch - 1) / kStepsPerLaunch + 1));
-    auto key = std::make_tuple(kind, -(long)launches, b, ctx->cap, 1ULL);
-    auto it = ctx->graphs.find(key);
-    if (it == ctx->graphs.end()) {
-      GraphEntry ge;
-      if ((rc = capture_steps_graph(ctx, kind, b, launches, ge))) return rc;
-      it = ctx->graphs.emplace(key, ge).first;
-    }
-    CR_TRY(cudaGraphLaunch(it->second.exec, ctx->stream));
-    ctx->launches += it->second.launches;
+    if ((rc = launch_steps(ctx, kind, b, launches))) return rc;
     if ((rc = read_status(ctx))) return rc;
     const DevStatus& st = *ctx->status_h;
     if (st.abort) {

@@ -68,5 +68,5 @@ def test_coordinates_far_out(cuda_device, boxes):
 
 @pytest.mark.parametrize("nv,lanes", [(96, 2), (95, 2), (128, 1), (3, 1), (3, 2)])
 def test_ring_sizes(cuda_device, nv, lanes):
-    pk = synth.make_packing([nv] * 9, [1.0] * 9, 1.05, 0.35, seed=8, placement="rsa")
+    pk = synth.make_packing([nv] * 9, [1.0] * 9, 1.05, 0.35 if nv > 10 else 0.06, seed=8, placement="rsa")
     _same(_states(pk, "wca", "vertexSmooth", lanes, dt=2e-4))
