@@ -11,6 +11,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cr_fire.cuh"
 #include "cr_launch.h"
 #include "cr_tile.cuh"
 
@@ -151,7 +152,7 @@ struct cr_ctx {
   bool degraded = false;
   // state at the start of a multi-step sequence, restored if a barrier gives up
   double2 *snap_pos = nullptr, *snap_vel = nullptr, *snap_force = nullptr, *snap_last = nullptr;
-  double* snap_angle = nullptr;
+  double *snap_angle = nullptr, *snap_fire = nullptr;
 
   std::map<std::tuple<int, long, int, int, unsigned long long>, GraphEntry> graphs;
 
@@ -724,13 +725,14 @@ int launch_steps(cr_ctx* ctx, int kind, int b, int launches) {
 int run_ops(cr_ctx* ctx, int kind, long nsteps);
 
 // The state a multi-step sequence starts from (positions, velocities,
-// forces, last-build positions, self-propulsion angles), saved or restored.
+// forces, last-build positions, self-propulsion angles, FIRE scalars), saved or
+// restored.
 int sequence_state(cr_ctx* ctx, int b, bool restore) {
   int rc;
   if (!ctx->snap_pos) {
     if ((rc = dalloc(ctx, &ctx->snap_pos, ctx->nv)) || (rc = dalloc(ctx, &ctx->snap_vel, ctx->nv)) ||
         (rc = dalloc(ctx, &ctx->snap_force, ctx->nv)) || (rc = dalloc(ctx, &ctx->snap_last, ctx->nv)) ||
-        (rc = dalloc(ctx, &ctx->snap_angle, ctx->np)))
+        (rc = dalloc(ctx, &ctx->snap_angle, ctx->np)) || (rc = dalloc(ctx, &ctx->snap_fire, 8)))
       return rc;
   }
   const size_t v2 = (size_t)ctx->nv * sizeof(double2), pa = (size_t)ctx->np * sizeof(double);
@@ -741,6 +743,8 @@ int sequence_state(cr_ctx* ctx, int b, bool restore) {
                            ctx->stream));
   CR_TRY(cudaMemcpyAsync(restore ? ctx->p_angle : ctx->snap_angle, restore ? ctx->snap_angle : ctx->p_angle, pa,
                          cudaMemcpyDeviceToDevice, ctx->stream));
+  CR_TRY(cudaMemcpyAsync(restore ? ctx->fire_state : ctx->snap_fire, restore ? ctx->snap_fire : ctx->fire_state,
+                         8 * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
   return CR_OK;
 }
 
@@ -758,6 +762,7 @@ int rerun_degraded(cr_ctx* ctx, int b0, const DevStatus& start, int kind, long n
   s.done_ctr = s.bar_count = s.pbar = 0;
   s.pflag[0] = 0;
   s.pbase = s.steps_left = 0;
+  s.bpending = 0;
   *ctx->status_h = s;
   if ((rc = upload(ctx, ctx->status, ctx->status_h, sizeof(DevStatus)))) return rc;
   enter_degraded(ctx);
@@ -819,6 +824,71 @@ int run_steps(cr_ctx* ctx, int kind, long nsteps) {
   return CR_OK;
 }
 
+// FIRE iterations in k_fire_steps launches, each followed by the one-launch
+// build, until the device's count of iterations left reaches zero or the
+// force tolerance is met; the launches are sized and recovered as those of
+// run_steps.
+FireStepsFn fire_steps_eligible(cr_ctx* ctx, int kind) {
+  if (kind != KIND_FIRE || !ctx->multistep || !ctx->use_graphs || ctx->shape == CR_SHAPE_RIGID) return nullptr;
+  if (ctx->precision != CR_PRECISION_FP64 || ctx->particle == CR_PARTICLE_ACTIVE) return nullptr;
+  FireStepsFn fn = fire_steps_fn(ctx->potential, inter_kind(ctx), ctx->lanes);
+  return fire_steps_max_blocks(fn, ctx->lanes) >= (int)ctx->tiles_h.size() ? fn : nullptr;
+}
+
+int run_fire_steps(cr_ctx* ctx, FireStepsFn fn, long nsteps) {
+  int rc;
+  const int b = ctx->cur;
+  if ((rc = sequence_state(ctx, b, false))) return rc;
+  ctx->status_h->steps_left = nsteps;
+  ctx->status_h->bpending = 0;
+  const DevStatus start = *ctx->status_h;  // read by the caller's clear_flags
+  if ((rc = upload(ctx, ctx->status, ctx->status_h, sizeof(DevStatus)))) return rc;
+  long long left = nsteps;
+  for (;;) {
+    StepArgs s = base_args(ctx);
+    s.kind = KIND_FIRE;
+    s.pos_out = ctx->pos[b];
+    s.accumulate = 1;
+    s.write_out = 1;
+    s.fire_tol = ctx->fp.tol;
+    s.persist_max = kStepsPerLaunch;
+    LaunchCfg c = tile_cfg(ctx);
+    c.pdl = true;
+    NbrArgs nb = nbr_args(ctx, b, ctx->cut_distance);
+    nb.count_update = 1;
+    const int launches =
+        (int)std::min<long long>(kStepsLaunches, std::max<long long>(2, (left + kStepsPerLaunch - 1) / kStepsPerLaunch + 1));
+    for (int r = 0; r < launches; r++) {
+      CR_TRY(launch_fire_steps(fn, c, ctx->p, arrays(ctx, b), s, ctx->fp, ctx->fire_state));
+      launch_nbr_fused(ctx->stream, ctx->p, ctx->grid, nb, nbr_fused_blocks(ctx->nv, ctx->fused_max), 0, true);
+      ctx->launches += 2;
+    }
+    CR_TRY(cudaGetLastError());
+    if ((rc = read_status(ctx))) return rc;
+    const DevStatus& st = *ctx->status_h;
+    if (st.abort) {
+      if (st.stalled) return rerun_degraded(ctx, b, start, KIND_FIRE, nsteps);
+      if (st.nonfinite) return ctx->fail(CR_ENONFINITE, "non-finite force during the step sequence");
+      if (!st.overflow) return ctx->fail(CR_ECUDA, "step sequence aborted");
+      // a rebuild found more neighbours than capacity: grow the list, rebuild
+      // from the positions the failed build read, count the update and carry
+      // on with the pending force op
+      if ((rc = clear_flags(ctx))) return rc;
+      ctx->cap = 0;
+      if ((rc = build_list(ctx, b, ctx->cut_distance))) return rc;
+      if ((rc = clear_flags(ctx))) return rc;
+      ctx->status_h->update_count += 1;
+      if ((rc = upload(ctx, ctx->status, ctx->status_h, sizeof(DevStatus)))) return rc;
+      continue;
+    }
+    if (st.steps_left <= 0 || st.converged) break;
+    left = st.steps_left;
+  }
+  if (ctx->status_h->max_ever > 0)
+    ctx->list_size_ref = std::max<long long>(ctx->list_size_ref, pow2ceil(ctx->status_h->max_ever));
+  return CR_OK;
+}
+
 // Runs nsteps integrator steps (or FIRE iterations) as chunks of captured
 // graphs.  Non-FIRE chunks are launched back to back with one status read at
 // the end; FIRE reads the status after every chunk to stop at convergence.
@@ -843,6 +913,7 @@ int run_ops(cr_ctx* ctx, int kind, long nsteps) {
   }
   if ((rc = clear_flags(ctx))) return rc;
   if (steps_eligible(ctx, kind, nsteps)) return run_steps(ctx, kind, nsteps);
+  if (FireStepsFn fn = fire_steps_eligible(ctx, kind)) return run_fire_steps(ctx, fn, nsteps);
   const long chunk = 128;
   std::vector<std::vector<Op>> plan;
   std::vector<long> sizes;
@@ -1088,7 +1159,7 @@ int cr_destroy(cr_ctx* ctx) {
                   ctx->p_torque, ctx->p_moi, ctx->v_torque, ctx->sp_angle, ctx->block_sum, ctx->cell_bucket, ctx->bucket_pos, ctx->bucket_rad,
                   ctx->bucket_ring, ctx->bucket_pq,
                   ctx->prad, ctx->plast, ctx->pid, ctx->pnbr, ctx->pnbr_cnt, ctx->pstatus, ctx->pfire, ctx->pdraws,
-                  ctx->snap_pos, ctx->snap_vel, ctx->snap_force, ctx->snap_last, ctx->snap_angle};
+                  ctx->snap_pos, ctx->snap_vel, ctx->snap_force, ctx->snap_last, ctx->snap_angle, ctx->snap_fire};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (ctx->status_h) cudaFreeHost(ctx->status_h);

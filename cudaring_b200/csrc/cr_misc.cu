@@ -1,4 +1,5 @@
 // Per-vertex update kernels and reductions around the tiled force kernel.
+#include "cr_fire.cuh"
 #include "cr_launch.h"
 #include "cr_tile.cuh"
 
@@ -69,10 +70,7 @@ __global__ void __launch_bounds__(256) k_drift(const __grid_constant__ SysParams
 }
 
 // FIRE iteration up to the position update (FIRE::minimizerVertexLoop,
-// src/FIRE.cu:397-406): checkFIREParams (:338-371) from P = v.F, the
-// half kick (:320-335), bendVertexVelocityTowardsForce (:374-394) and
-// updateVertexPosition (:302-317).  |v|^2 after the half kick is formed from
-// the three sums of the previous force op:  |v + h F|^2 = vv + 2h vF + h^2 FF.
+// src/FIRE.cu:397-406), one vertex per thread (fire_next, fire_move).
 __global__ void __launch_bounds__(256) k_fire_pre(const __grid_constant__ SysParams p,
                                                   const __grid_constant__ SysArrays a,
                                                   const __grid_constant__ StepArgs s,
@@ -81,45 +79,19 @@ __global__ void __launch_bounds__(256) k_fire_pre(const __grid_constant__ SysPar
   DevStatus* st = s.status;
   const long long it = st->fire_iters;
   const double* cur = fire_state + (it & 1) * 4;
-  double dt = cur[0], alpha = cur[1];
-  long long nstep = (long long)cur[2];
+  FireScalars f{cur[0], cur[1], (long long)cur[2]};
   const double P = st->sums[S_VF], vv = st->sums[S_VV], ff = st->sums[S_FF];
-  bool rollback = false;
-  if (P > 0) {
-    nstep++;
-    if (nstep > fp.min_step) {
-      dt = fmin(dt * fp.f_inc, fp.dt_max);
-      alpha *= fp.f_a;
-    }
-  } else {
-    nstep = 0;
-    dt = fmax(dt * fp.f_dec, fp.dt_max / 10);
-    alpha = fp.a_start;
-    rollback = true;
-  }
+  const bool rollback = fire_next(fp, P, f);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     double* nxt = fire_state + ((it + 1) & 1) * 4;
-    nxt[0] = dt;
-    nxt[1] = alpha;
-    nxt[2] = (double)nstep;
+    nxt[0] = f.dt;
+    nxt[1] = f.alpha;
+    nxt[2] = (double)f.nstep;
   }
-  const double h = 0.5 * dt;
-  const double vpost2 = rollback ? (h * h) * ff : vv + dt * P + (h * h) * ff;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v < p.nv) {
-    double2 x = a.pos[v];
-    double2 vel = s.vel[v];
-    const double2 f = s.force[v];
-    if (rollback) {
-      x = make_double2(x.x - h * vel.x, x.y - h * vel.y);
-      vel = make_double2(0.0, 0.0);
-    }
-    vel = make_double2(vel.x + h * f.x, vel.y + h * f.y);
-    if (ff > 0) {
-      const double ratio = sqrt(vpost2 / ff);
-      vel = make_double2((1 - alpha) * vel.x + alpha * f.x * ratio, (1 - alpha) * vel.y + alpha * f.y * ratio);
-    }
-    x = make_double2(x.x + dt * vel.x, x.y + dt * vel.y);
+    double2 x = a.pos[v], vel = s.vel[v];
+    fire_move(f, rollback, P, vv, ff, s.force[v], x, vel);
     s.pos_out[v] = x;
     s.vel[v] = vel;
     if (3.0 * dist_of(pbc2(p, x, s.last_pos[v])) > s.disp_cutoff) st->rebuild = 1;

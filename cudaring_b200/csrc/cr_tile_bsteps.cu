@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
         break;
       }
     }
-    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, true, 2>(p, a, s, a.pos, s.pos_out, 0ull, nullptr, false, &g, tile);
+    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, true, 2>(p, a, s, a.pos, s.pos_out, 0ull, nullptr, j > 0, &g, tile);
     if (steps_barrier(st) < 0) {
       stalled = true;
       break;

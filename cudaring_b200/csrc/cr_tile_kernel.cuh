@@ -789,12 +789,14 @@ __device__ __forceinline__ void join_first(int sync) {
 // force reported in *pflag instead of the status block, whether the loop is
 // to end after this step (a rebuild is due, a force is not finite) returned,
 // and the last-block protocol left to the caller; 2 the persistent batched
-// FIRE kernel: plain position loads, everything else as for one op.
+// FIRE kernel: plain position loads, everything else as for one op; 3 the FIRE
+// kernel of one system: the CTA's partial sums are all it leaves (fire_hdt:
+// half the time step).  reuse: not the kernel's first op.
 template <int POT, int INTER, int MODE, int BLOCK, int L, int PREC, bool BATCH, int PERSIST>
 __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a, const StepArgs& s,
                                           const double2* __restrict__ pin, double2* __restrict__ pout,
                                           unsigned long long step, int* pflag, bool reuse,
-                                          const Stage<BLOCK / L>* g, const int4& tile) {
+                                          const Stage<BLOCK / L>* g, const int4& tile, double fire_hdt = 0.0) {
   constexpr int TV = BLOCK / L;
   // the multi-step kernel stores no energies and no sums (its ops run with
   // write_out = accumulate = 0), so its energy terms are left out at compile time
@@ -858,13 +860,19 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
   if (t < nvt) {
     const int v = v0 + t;
     int2 tp;
-    if (PERSIST == 1 && reuse) {
-      // a later step of the multi-step kernel: the CTA holds the same tile,
-      // so its topology, rest lengths and angles, last-build positions and its
-      // own positions and velocities (stored by the last step's tail) are
-      // still in shared memory
+    // a later op of a persistent kernel: the CTA holds the same tile, so its
+    // topology, rest lengths and angles and last-build positions are still in
+    // shared memory; in the multi-step kernel so are its own positions and
+    // velocities (stored by the last step's tail), the FIRE kernels' pre-kick
+    // has stored new ones
+    if (PERSIST != 0 && reuse) {
       tp = s_tp[t];
       a0r = s_a0[t];
+      if constexpr (PERSIST != 1) {
+        cp_async16(&s_vel[t], s.vel + v);
+        cp_async_commit();
+        s_pos[t] = ld_pos<true>(pin + v);
+      }
     } else {
       if constexpr (MODE == MODE_STEP) {
         cp_async16(&s_vel[t], s.vel + v);
@@ -879,7 +887,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
       s_th0[t] = __ldg(a.theta0 + v);
       a0r = __ldg(a.a0 + tp.x);
       s_tp[t] = tp;
-      if constexpr (PERSIST == 1) s_a0[t] = a0r;
+      if constexpr (PERSIST != 0) s_a0[t] = a0r;
     }
     ring = tp.x;
     k = tp.y & 0xffff;
@@ -1273,6 +1281,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
       double hdt = s.hdt;
       if (s.kind == KIND_FIRE) {
         if constexpr (BATCH) hdt = 0.5 * s.bfire_state[(sysid * 2 + ((s.bsys[sysid].fire_iters + 1) & 1)) * 4];
+        else if constexpr (PERSIST == 3) hdt = fire_hdt;
         else hdt = 0.5 * s.fire_state[((st->fire_iters + 1) & 1) * 4];
       }
       const double dcut = BATCH ? s.bsys[sysid].disp_cutoff : s.disp_cutoff;
@@ -1361,6 +1370,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     if (kOut && s.accumulate) {
       // per-CTA partials in a fixed order, compensated
       block_partials<BLOCK>(sums, s_red, s.partials + (size_t)blockIdx.x * NSUM);
+      if constexpr (PERSIST == 3) return false;  // the caller reduces them
     } else if constexpr (PERSIST == 1) {
       if (nonfinite) *(volatile int*)pflag = 1;
       return __syncthreads_or(nonfinite | stop) != 0;
