@@ -112,6 +112,14 @@ struct cr_ctx {
   double* diff_area = nullptr; // [np][4] hyper-dual ring areas
   CgState* cg_state = nullptr;
   double* cg_part = nullptr;   // [148][8] CG reduction partials
+  // many iterations per launch (k_cg_steps): pair blocks at list capacity
+  // cgs_cap, tiles, p of the last iteration; cleared when a barrier gave up
+  double2 *cgs_kxy = nullptr, *cgs_p = nullptr;
+  double* cgs_kyy = nullptr;
+  int* cgs_kj = nullptr;
+  int2* cgs_tiles = nullptr;
+  int cgs_cap = 0, cgs_block = 0, cgs_ntiles = 0;
+  bool cg_steps = true;
   double* cg_minv = nullptr;   // [nv][3] inverse diagonal Hessian blocks (block-Jacobi preconditioner)
   int cg_precond = 1;          // 1: block-Jacobi preconditioner in cr_hessian_solve; 0: none
   int partials_n = 0;
@@ -1155,7 +1163,7 @@ int cr_destroy(cr_ctx* ctx) {
                   ctx->cell_cnt, ctx->cell_start, ctx->cell_vid, ctx->cell_ring, ctx->cell_pos, ctx->cell_rad,
                   ctx->partials, ctx->status, ctx->fire_state, ctx->p_vel, ctx->p_force, ctx->p_angvel,
                   ctx->diff_f, ctx->diff_e, ctx->diff_dot, ctx->diff_vec, ctx->diff_area, ctx->cg_state,
-                  ctx->cg_part, ctx->cg_minv,
+                  ctx->cg_part, ctx->cg_minv, ctx->cgs_kxy, ctx->cgs_kyy, ctx->cgs_kj, ctx->cgs_tiles, ctx->cgs_p,
                   ctx->p_torque, ctx->p_moi, ctx->v_torque, ctx->sp_angle, ctx->block_sum, ctx->cell_bucket, ctx->bucket_pos, ctx->bucket_rad,
                   ctx->bucket_ring, ctx->bucket_pq,
                   ctx->prad, ctx->plast, ctx->pid, ctx->pnbr, ctx->pnbr_cnt, ctx->pstatus, ctx->pfire, ctx->pdraws,
@@ -2145,44 +2153,20 @@ static int diff_energy(cr_ctx* ctx, double out[4]) {
   return CR_OK;
 }
 
-static int dev_dot(cr_ctx* ctx, const double* a, const double* b, int n, double* out) {
-  const int nb = std::min(256, std::max(1, (n + 255) / 256));
-  launch_dot_partials(ctx->stream, n, a, b, ctx->diff_dot, nb);
-  ctx->launches++;
-  double part[256];
-  int rc = download(ctx, part, ctx->diff_dot, nb * sizeof(double));
-  if (rc) return rc;
-  double s = 0.0;
-  for (int i = 0; i < nb; i++) s += part[i];
-  *out = s;
-  return CR_OK;
-}
-
-static int dev_project(cr_ctx* ctx, double* x) {
-  std::vector<double> h((size_t)2 * ctx->nv);
-  int rc = download(ctx, h.data(), x, h.size() * sizeof(double));
-  if (rc) return rc;
-  double mx = 0.0, my = 0.0;
-  for (int v = 0; v < ctx->nv; v++) {
-    mx += h[2 * v];
-    my += h[2 * v + 1];
-  }
-  launch_sub_mean(ctx->stream, ctx->nv, x, mx / ctx->nv, my / ctx->nv);
-  ctx->launches++;
-  CR_TRY(cudaGetLastError());
-  return CR_OK;
-}
-
 extern "C" int cr_hvp_device(cr_ctx* ctx, const double* v_dev, double* hv_dev) {
   if (!ctx || !v_dev || !hv_dev) return CR_EINVAL;
   int rc;
   if ((rc = diff_ready(ctx))) return rc;
   DiffArgs g = diff_args(ctx);
   g.t1 = reinterpret_cast<const double2*>(v_dev);
+  // straight into the caller's array unless that overlaps v or is not aligned
+  // for two doubles
+  const size_t bytes = (size_t)2 * ctx->nv * sizeof(double);
+  const char *vb = reinterpret_cast<const char*>(v_dev), *hb = reinterpret_cast<const char*>(hv_dev);
+  const bool direct = (hb + bytes <= vb || vb + bytes <= hb) && (size_t)hb % sizeof(double2) == 0;
+  g.hv_out = reinterpret_cast<double2*>(direct ? hv_dev : ctx->diff_f);
   if ((rc = diff_launch(ctx, g))) return rc;
-  launch_extract_hv(ctx->stream, ctx->nv, ctx->diff_f, hv_dev);
-  ctx->launches++;
-  CR_TRY(cudaGetLastError());
+  if (!direct) CR_TRY(cudaMemcpyAsync(hv_dev, ctx->diff_f, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
   CR_TRY(cudaStreamSynchronize(ctx->stream));
   return CR_OK;
 }
@@ -2245,6 +2229,57 @@ extern "C" int cr_param_derivatives(cr_ctx* ctx, int param, double* dU, double* 
   return CR_OK;
 }
 
+// Scratch and tiles of k_cg_steps; *ok = false where it does not apply (smooth
+// interaction, a grid the GPU does not hold at once, a barrier that gave up
+// before).
+static int cg_steps_ready(cr_ctx* ctx, bool* ok) {
+  *ok = false;
+  if (!ctx->cg_steps || ctx->degraded || inter_kind(ctx) != INT_VV) return CR_OK;
+  int rc;
+  if (!ctx->cgs_tiles) {
+    // the smallest CTA whose grid gives each SM at most one (a few thousand
+    // vertices then use every SM, and the sums over the grid stay short); for
+    // larger systems the grid of the fewest CTAs that the GPU holds at once
+    std::vector<int2> tiles;
+    int sms = 0;
+    CR_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    for (int block : {64, 96, 128}) {
+      std::vector<int2> cut;
+      bool fits = true;
+      for (int q = 0; q < ctx->np && fits;) {
+        const int first = ctx->ring_first_h[q];
+        int end = first;
+        while (q < ctx->np && end + ctx->ring_nv_h[q] - first <= block) end += ctx->ring_nv_h[q++];
+        fits = end > first;
+        cut.push_back(make_int2(first, end));
+      }
+      if (!fits || cg_steps_max_blocks(ctx->potential, block) < (int)cut.size()) continue;
+      if (tiles.empty() || cut.size() < tiles.size()) {
+        tiles = cut;
+        ctx->cgs_block = block;
+      }
+      if ((int)tiles.size() <= sms) break;
+    }
+    if (tiles.empty()) return CR_OK;
+    ctx->cgs_ntiles = (int)tiles.size();
+    if ((rc = dalloc(ctx, &ctx->cgs_p, (size_t)2 * ctx->nv)) ||
+        (rc = dalloc(ctx, &ctx->cg_part, (size_t)8 * std::max(148, ctx->cgs_ntiles))) ||
+        (rc = dalloc(ctx, &ctx->cgs_tiles, tiles.size())) ||
+        (rc = upload(ctx, ctx->cgs_tiles, tiles.data(), tiles.size() * sizeof(int2))))
+      return rc;
+  }
+  if (cg_steps_max_blocks(ctx->potential, ctx->cgs_block) < ctx->cgs_ntiles) return CR_OK;
+  if (ctx->cgs_cap < ctx->cap) {
+    const size_t n = (size_t)ctx->cap * ctx->nv;
+    if ((rc = dalloc(ctx, &ctx->cgs_kxy, n)) || (rc = dalloc(ctx, &ctx->cgs_kyy, n)) ||
+        (rc = dalloc(ctx, &ctx->cgs_kj, n)))
+      return rc;
+    ctx->cgs_cap = ctx->cap;
+  }
+  *ok = true;
+  return CR_OK;
+}
+
 extern "C" int cr_hessian_solve(cr_ctx* ctx, const double* b, double* x, double tol, long maxIter, long* iters,
                                 double* relres) {
   if (!ctx || !b || !x || maxIter < 0) return CR_EINVAL;
@@ -2273,42 +2308,51 @@ extern "C" int cr_hessian_solve(cr_ctx* ctx, const double* b, double* x, double 
     minv = ctx->cg_minv;
   }
   if ((rc = upload(ctx, r, b, (size_t)n * sizeof(double)))) return rc;
-  if ((rc = dev_project(ctx, r))) return rc;
-  CR_TRY(cudaMemsetAsync(xd, 0, (size_t)n * sizeof(double), ctx->stream));
-  launch_cg_apply(ctx->stream, ctx->nv, minv, r, zv);
-  CR_TRY(cudaGetLastError());
-  if ((rc = dev_project(ctx, zv))) return rc;
-  CR_TRY(cudaMemcpyAsync(pv, zv, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-  double bb, rz;
-  if ((rc = dev_dot(ctx, r, r, n, &bb)) || (rc = dev_dot(ctx, r, zv, n, &rz))) return rc;
-  CgState cs;
-  memset(&cs, 0, sizeof(cs));
-  cs.rr = bb;
-  cs.bb = bb;
-  cs.rz = rz;
-  cs.tol = tol;
-  cs.max_iters = maxIter;
-  cs.done = (maxIter == 0 || !(bb > 0.0) || !(std::sqrt(cs.rr / bb) > tol)) ? 1 : 0;
-  if ((rc = upload(ctx, ctx->cg_state, &cs, sizeof(cs)))) return rc;
-  // the iterations run in captured chunks: H p (hyper-dual forces along p),
-  // then the CG scalars and vector updates, all on the device; every kernel
-  // returns at once after the state says done, so a chunk may overrun
-  constexpr int kChunk = 32;
-  DiffArgs g = diff_args(ctx);
-  g.t1 = reinterpret_cast<const double2*>(pv);
-  g.skip = &ctx->cg_state->done;
   CgArgs a;
   a.nv = ctx->nv;
   a.x = xd;
   a.r = r;
   a.p = pv;
   a.hp = hp;
-  a.fhd = ctx->diff_f;
   a.st = ctx->cg_state;
-  a.partials = ctx->cg_part;
-  a.nblk = cg_blocks(ctx->nv);
   a.z = zv;
   a.minv = minv;
+  a.partials = ctx->cg_part;
+  a.nblk = cg_blocks(ctx->nv);
+  launch_cg_start(ctx->stream, a, tol, maxIter);
+  ctx->launches++;
+  CR_TRY(cudaGetLastError());
+  CgState cs;
+  if ((rc = download(ctx, &cs, ctx->cg_state, sizeof(cs)))) return rc;
+  bool many = false;
+  if (!cs.done && (rc = cg_steps_ready(ctx, &many))) return rc;
+  if (many) {
+    // launches of up to kLaunch iterations each until the state says done
+    constexpr int kLaunch = 4096;
+    a.partials = ctx->cg_part;  // cg_steps_ready may have made it larger
+    if ((rc = read_status(ctx))) return rc;
+    CgSteps ks{ctx->cgs_kxy, ctx->cgs_kyy, ctx->cgs_kj, ctx->cgs_tiles, ctx->cgs_ntiles,
+               {ctx->cgs_p, ctx->cgs_p + ctx->nv}, ctx->status_h->spin_limit, kLaunch};
+    while (!cs.done && !cs.stalled) {
+      CR_TRY(launch_cg_steps(ctx->stream, ctx->potential, ctx->cgs_block, diff_args(ctx), a, ks));
+      ctx->launches++;
+      if ((rc = download(ctx, &cs, ctx->cg_state, sizeof(cs)))) return rc;
+    }
+    if (cs.stalled) {
+      // the GPU did not hold every CTA at once: the whole solve again with one
+      // launch per op, now and from here on
+      ctx->cg_steps = false;
+      return cr_hessian_solve(ctx, b, x, tol, maxIter, iters, relres);
+    }
+  }
+  // otherwise the iterations run in captured chunks: H p (dual forces along p),
+  // then the CG scalars and vector updates, all on the device; every kernel
+  // returns at once after the state says done, so a chunk may overrun
+  constexpr int kChunk = 32;
+  DiffArgs g = diff_args(ctx);
+  g.t1 = reinterpret_cast<const double2*>(pv);
+  g.skip = &ctx->cg_state->done;
+  g.hv_out = reinterpret_cast<double2*>(hp);
   cudaGraphExec_t exec = nullptr;
   if (!cs.done) {
     cudaGraph_t graph = nullptr;
@@ -2336,7 +2380,7 @@ extern "C" int cr_hessian_solve(cr_ctx* ctx, const double* b, double* x, double 
   CR_TRY(cudaGetLastError());
   if (cs.bad) return ctx->fail(CR_ENONFINITE, "Hessian not positive along a CG direction");
   if (iters) *iters = (long)cs.iters;
-  if (relres) *relres = bb > 0.0 ? std::sqrt(cs.rr / bb) : 0.0;
+  if (relres) *relres = cs.bb > 0.0 ? std::sqrt(cs.rr / cs.bb) : 0.0;
   return download(ctx, x, xd, (size_t)n * sizeof(double));
 }
 

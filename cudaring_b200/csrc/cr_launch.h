@@ -98,6 +98,7 @@ struct DiffArgs {
   const int* nbr_cnt;
   int nbr_cap;
   double* force_out;   // [nv][8]: Fx (a, b, c, d), Fy (a, b, c, d)
+  double2* hv_out;     // nullable: only -(e1 part of F) is wanted (t1 set, every other tangent zero)
   double* energy_out;  // [nv][4]
   double* ring_area;   // [np][4] scratch: hyper-dual ring areas (filled by the launch)
   const int* skip;     // nullable: nothing is evaluated while *skip != 0
@@ -116,6 +117,8 @@ struct CgState {
   double mx, my;          // mean of H p over the vertices (removed: translations)
   long long iters, max_iters;
   int done;               // converged, iteration limit, or non-positive curvature
+  unsigned long long bar; // grid barrier of k_cg_steps: arrivals
+  int stalled;            // one of its waits gave up
   int bad;                // 1: a non-positive curvature p.Hp was met
   double rz;              // r.z with z = M^-1 r (the preconditioned residual; = |r|^2 without one)
   double zx, zy;          // mean of z over the vertices (removed: translations)
@@ -126,7 +129,6 @@ struct CgArgs {
   double* r;
   double* p;
   double* hp;
-  const double* fhd;  // hyper-dual forces of the H p launch
   CgState* st;
   double* partials;   // [nblk][8]
   int nblk;
@@ -134,16 +136,30 @@ struct CgArgs {
   const double* minv; // [nv][3] inverse diagonal blocks (a, b, d of [[a, b], [b, d]]); null: no preconditioner
 };
 void launch_cg_iteration(cudaStream_t st, const CgArgs& a);
+// Many iterations in one launch (vertex-vertex interaction; cr_diff.cu).
+// Scratch: the stiffness blocks of the pairs in range, [cap][nv] (xx, xy), yy
+// and the neighbour; tiles (first, end vertex) of whole rings, at most
+// as many vertices each as a CTA has threads (64, 96 or 128); p of the last iteration, two
+// buffers.
+struct CgSteps {
+  double2* kxy;
+  double* kyy;
+  int* kj;
+  const int2* tiles;
+  int ntiles;
+  double2* pold[2];
+  long long spin_limit;
+  int max_iters;   // iterations a launch makes at most
+};
+int cg_steps_max_blocks(int pot, int block);          // CTAs the device holds at once
+cudaError_t launch_cg_steps(cudaStream_t st, int pot, int block, const DiffArgs& g, const CgArgs& a, const CgSteps& k);
 // Block-Jacobi preconditioner from a diag-mode hyper-dual launch: minv[v] the
 // inverse of the vertex's 2 x 2 Hessian block (its positive part where the
-// block is not positive definite); z = M^-1 r.
+// block is not positive definite).  launch_cg_start: the solve's first
+// vectors and state from b in a.r.
 void launch_cg_prec(cudaStream_t st, int nv, const double* fhd, double* minv);
-void launch_cg_apply(cudaStream_t st, int nv, const double* minv, const double* r, double* z);
+void launch_cg_start(cudaStream_t st, const CgArgs& a, double tol, long long max_iters);
 int cg_blocks(int nv);
-void launch_dot_partials(cudaStream_t st, int n, const double* a, const double* b, double* out, int nblocks);
-void launch_axpby(cudaStream_t st, int n, double a, const double* x, double b, double* y);
-void launch_extract_hv(cudaStream_t st, int nv, const double* fhd, double* hv);
-void launch_sub_mean(cudaStream_t st, int nv, double* x, double mx, double my);
 
 // cr_nbr.cu
 // Vertex ids a cell bucket of the one-launch build holds; a build that finds
