@@ -8,8 +8,8 @@
 // cell-list build, which rebuilds only the systems whose displacement check
 // fired.  Each system keeps its own FIRE scalars, convergence flag and
 // rebuild flag; a converged system's tiles exit at once, so an iteration
-// costs what the unconverged systems cost.  Iterations run as captured CUDA
-// graphs with one conditional rebuild node per iteration.
+// costs what the unconverged systems cost.  Every pre-kick is followed by the
+// two build kernels, which return at once unless a system was flagged.
 //
 // On top runs the quasi-static compression protocol of the reference's
 // compressFIRE driver (compressFIRE.cpp:101-205), per system: FIRE to the
@@ -41,7 +41,7 @@ struct CompSys {
 
 struct cr_batch {
   int device = 0;
-  cudaStream_t stream = nullptr, side = nullptr;
+  cudaStream_t stream = nullptr;
   int S = 0, nv = 0, np = 0;
   std::vector<int> sys_np, sys_nv, sys_v0, sys_r0;  // per system: rings, vertices, first vertex, first ring
   std::vector<int> ring_nv_h, ring_first_h, ring_sys_h, vsys_h;
@@ -100,8 +100,6 @@ struct cr_batch {
   // grid-barrier wait gave up; the chunk graph of the current list capacity
   bool no_persist = false;
   std::map<BFireStepsFn, int> persist_max;  // CTAs each kernel holds resident at once
-  cudaGraphExec_t pchunk = nullptr;
-  std::map<std::pair<long, int>, cudaGraphExec_t> graphs;  // (iterations, cap) -> FIRE chunk
   long long launches = 0;
   std::string err;
   int fail(int code, const std::string& m) {
@@ -143,6 +141,7 @@ struct BNbr {
   int* cell_ring;
   int* cell_pq;
   const int4* sgrid;
+  const int* sys_v0;
   BatchSys* bsys;
   DevStatus* status;
   int S;
@@ -160,39 +159,85 @@ __device__ __forceinline__ int b_cell_coord(double x, double L, double invL, int
   return c < 0 ? 0 : (c >= nc ? nc - 1 : c);
 }
 
-__global__ void k_bguard(DevStatus* st) {
-  if (threadIdx.x == 0) {
-    st->overflow = 0;
-    st->max_count = 0;
-  }
+// Both build kernels follow every op that may flag a system and return at once
+// when none is flagged (two early exits cost less than a conditional graph
+// node, and sequences of ops need no graph).
+__device__ __forceinline__ bool b_nothing_due(const BNbr& n) {
+  if (n.all) return false;
+  const volatile DevStatus* st = n.status;
+  return !st->rebuild || st->abort;
 }
 
-__global__ void __launch_bounds__(256) k_bcell_count(const __grid_constant__ BNbr n) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n.nv) return;
-  const int s = n.vsys[v];
+// The cells of a system, by one CTA: counts, starts (the entries of system s
+// are its vertices' own range, its starts begin at its first cell + s, one more
+// than its cells), and its vertices in cell order, ascending ids inside a
+// cell, with the data the search reads.  As count, scan, fill, sort and gather
+// kernels over all systems (the scan by one CTA over every cell of the batch)
+// this took most of a rebuild.
+__global__ void __launch_bounds__(1024) k_bcells(const __grid_constant__ BNbr n) {
+  if (b_nothing_due(n)) return;
+  const int s = blockIdx.x, t = threadIdx.x;
+  if (s == 0 && t == 0) {
+    n.status->overflow = 0;
+    n.status->max_count = 0;
+  }
   if (!b_selected(n, s)) return;
   const int4 g = n.sgrid[s];
   const Box bx = n.bsys[s].box;
-  const double2 x = n.pos[v];
-  const int cx = b_cell_coord(x.x, bx.lx, bx.inv_lx, g.x);
-  const int cy = b_cell_coord(x.y, bx.ly, bx.inv_ly, g.y);
-  const int c = g.z + cy * g.x + cx;
-  n.cell_of[v] = c;
-  n.slot[v] = atomicAdd(n.cell_cnt + c, 1);
-}
-
-__global__ void __launch_bounds__(256) k_bcell_fill(const __grid_constant__ BNbr n) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n.nv) return;
-  if (!b_selected(n, n.vsys[v])) return;
-  n.cell_vid[n.cell_start[n.cell_of[v]] + n.slot[v]] = v;
+  const int nc = g.x * g.y, v0 = n.sys_v0[s], v1 = s + 1 < n.S ? n.sys_v0[s + 1] : n.nv;
+  int* cnt = n.cell_cnt + g.z;
+  int* start = n.cell_start + g.z + s;
+  for (int c = t; c < nc; c += 1024) cnt[c] = 0;
+  __syncthreads();
+  for (int v = v0 + t; v < v1; v += 1024) {
+    const double2 x = n.pos[v];
+    const int c = b_cell_coord(x.y, bx.ly, bx.inv_ly, g.y) * g.x + b_cell_coord(x.x, bx.lx, bx.inv_lx, g.x);
+    n.cell_of[v] = g.z + c;
+    n.slot[v] = atomicAdd(cnt + c, 1);
+  }
+  __syncthreads();
+  // exclusive scan, a run of cells per thread
+  __shared__ int s_w[32];
+  const int per = (nc + 1023) / 1024, cb = min(nc, t * per), ce = min(nc, cb + per);
+  int sum = 0;
+  for (int c = cb; c < ce; c++) sum += __ldcg(cnt + c);
+  int incl = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((t & 31) >= o) incl += y;
+  }
+  if ((t & 31) == 31) s_w[t >> 5] = incl;
+  __syncthreads();
+  int run = v0 + incl - sum;
+  for (int w = 0; w < (t >> 5); w++) run += s_w[w];
+  for (int c = cb; c < ce; c++) {
+    start[c] = run;
+    run += __ldcg(cnt + c);
+  }
+  if (t == 0) start[nc] = v1;
+  __syncthreads();
+  for (int v = v0 + t; v < v1; v += 1024) n.cell_vid[start[n.cell_of[v] - g.z] + n.slot[v]] = v;
+  __syncthreads();
+  // every vertex to its start + the members of its cell with a smaller id; the
+  // ids in cell order go to slot, whose per-vertex slots are used up
+  for (int v = v0 + t; v < v1; v += 1024) {
+    const int c = n.cell_of[v] - g.z, b = start[c], e = start[c + 1];
+    int rank = 0;
+    for (int i = b; i < e; i++) rank += n.cell_vid[i] < v ? 1 : 0;
+    const int k = b + rank;
+    n.slot[k] = v;
+    n.cell_pos[k] = n.pos[v];
+    n.cell_rad[k] = n.rad[v];
+    n.cell_ring[k] = n.ring_of[v];
+    n.cell_pq[k] = n.pq_pack[v];
+  }
 }
 
 // The list rule of kernelCalcNeighborList (include/cudaKernel.cuh:1735-1763)
 // over the 3x3 stencil of the vertex's own system (one cell when the system
 // has fewer than three cells per side); the last CTA publishes the build.
 __global__ void __launch_bounds__(256) k_bnbr(const __grid_constant__ BNbr n) {
+  if (b_nothing_due(n)) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int cnt = 0;
   if (i < n.nv && b_selected(n, n.vsys[i])) {
@@ -213,14 +258,19 @@ __global__ void __launch_bounds__(256) k_bnbr(const __grid_constant__ BNbr n) {
         int xx = cx + dx;
         xx += (xx < 0) ? g.x : 0;
         xx -= (xx >= g.x) ? g.x : 0;
-        const int cc = g.z + yy * g.x + xx;
+        const int cc = g.z + s + yy * g.x + xx;
         const int kb = n.cell_start[cc], ke = n.cell_start[cc + 1];
         for (int k = kb; k < ke; k++) {
           if (n.cell_ring[k] == ring) continue;
-          const double d = dist_of(pbc2(bx, xi, n.cell_pos[k]));
-          if (-(1.0 - d / (ri + n.cell_rad[k])) < n.cut_distance) {
+          // the squares decide outside a relative band of 1e-9, the reference
+          // expression inside it
+          const double2 dl = pbc2(bx, xi, n.cell_pos[k]);
+          const double sq = fma(dl.y, dl.y, dl.x * dl.x), rsum = ri + n.cell_rad[k];
+          const double reach = (1.0 + n.cut_distance) * rsum, r2 = reach * reach;
+          const bool exact = !(n.cut_distance > -0.5) || (sq >= r2 * (1.0 - 1e-9) && sq <= r2 * (1.0 + 1e-9));
+          if (exact ? -(1.0 - sqrt(sq) / rsum) < n.cut_distance : sq < r2) {
             if (cnt < n.cap) {
-              n.nbr[(size_t)cnt * n.nv + i] = n.cell_vid[k];
+              n.nbr[(size_t)cnt * n.nv + i] = n.slot[k];
               n.nbr_pq[(size_t)cnt * n.nv + i] = n.cell_pq[k];
             }
             cnt++;
@@ -270,12 +320,6 @@ __global__ void __launch_bounds__(256) k_bfire_pre(const __grid_constant__ BFire
   DevStatus* st = f.st;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (!st->abort && v < f.nv) bfire_prekick(f, v);
-  if (is_last_block(st)) {
-    if (threadIdx.x == 0) {
-      st->done_ctr = 0;
-      if (f.use_cond) cudaGraphSetConditional(f.cond, (!st->abort && st->rebuild) ? 1u : 0u);
-    }
-  }
 }
 
 // Per-system sums of the stored velocities, forces and energies, one tile
@@ -589,7 +633,8 @@ int dalloc(cr_batch* b, T** p, size_t n) {
   if (n == 0) n = 1;
   cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
   if (e != cudaSuccess) return b->fail(CR_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  e = cudaMemset(*p, 0, n * sizeof(T));
+  // on the stream that uses the array: the default stream is not ordered with it
+  e = cudaMemsetAsync(*p, 0, n * sizeof(T), b->stream);
   if (e != cudaSuccess) return b->fail(CR_ECUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
   return CR_OK;
 }
@@ -607,12 +652,8 @@ int download(cr_batch* b, void* dst, const void* src, size_t bytes) {
 }
 
 void drop_graphs(cr_batch* b) {
-  for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
-  b->graphs.clear();
   if (b->comp_exec) cudaGraphExecDestroy(b->comp_exec);
   b->comp_exec = nullptr;
-  if (b->pchunk) cudaGraphExecDestroy(b->pchunk);
-  b->pchunk = nullptr;
 }
 
 int read_status(cr_batch* b) { return download(b, b->status_h, b->status, sizeof(DevStatus)); }
@@ -702,7 +743,7 @@ int setup_grids(cr_batch* b) {
   if (total > b->ncells_alloc) {
     drop_graphs(b);
     if ((rc = dalloc(b, &b->cell_cnt, total))) return rc;
-    if ((rc = dalloc(b, &b->cell_start, total + 1))) return rc;
+    if ((rc = dalloc(b, &b->cell_start, total + b->S + 1))) return rc;
     b->ncells_alloc = total;
   }
   return upload(b, b->sgrid, b->sgrid_h.data(), b->S * sizeof(int4));
@@ -732,6 +773,7 @@ BNbr nbr_args(cr_batch* b, int all) {
   n.cell_ring = b->cell_ring;
   n.cell_pq = b->cell_pq;
   n.sgrid = b->sgrid;
+  n.sys_v0 = b->sys_v0_d;
   n.bsys = b->bsys;
   n.status = b->status;
   n.S = b->S;
@@ -742,26 +784,9 @@ BNbr nbr_args(cr_batch* b, int all) {
 // The batched build as stream-ordered launches (capturable).
 void enqueue_build(cr_batch* b, cudaStream_t st, int all) {
   const BNbr n = nbr_args(b, all);
-  const int nb = (b->nv + 255) / 256;
-  k_bguard<<<1, 32, 0, st>>>(b->status);
-  k_bcell_count<<<nb, 256, 0, st>>>(n);
-  launch_cell_scan(st, b->ncells, b->cell_cnt, b->cell_start);
-  k_bcell_fill<<<nb, 256, 0, st>>>(n);
-  NbrArgs na{};
-  na.pos = b->pos;
-  na.rad = b->rad;
-  na.ring_of = b->ring_of;
-  na.cell_start = b->cell_start;
-  na.cell_vid = b->cell_vid;
-  na.cell_pos = b->cell_pos;
-  na.cell_rad = b->cell_rad;
-  na.cell_ring = b->cell_ring;
-  na.pq_pack = b->pq_pack;
-  na.nbr_pq = b->nbr_pq;
-  na.cell_pq = b->cell_pq;
-  launch_cell_sort(st, b->ncells, b->nv, na);
-  k_bnbr<<<nb, 256, 0, st>>>(n);
-  b->launches += 7;
+  k_bcells<<<b->S, 1024, 0, st>>>(n);
+  k_bnbr<<<(b->nv + 255) / 256, 256, 0, st>>>(n);
+  if (all) b->launches += 2;  // builds that only watch a sequence are not counted
 }
 
 int alloc_lists(cr_batch* b, int cap) {
@@ -881,7 +906,7 @@ int reduce_sys(cr_batch* b, int set_converged, cudaStream_t st = nullptr) {
 // One FIRE iteration over every unconverged system: pre-kick (with the
 // displacement check), conditional rebuild of the flagged systems, force +
 // second kick with per-system sums and convergence.
-BFire bfire_args(cr_batch* b, bool use_cond, cudaGraphConditionalHandle h) {
+BFire bfire_args(cr_batch* b) {
   BFire f;
   f.pos = b->pos;
   f.vel = b->vel;
@@ -894,28 +919,7 @@ BFire bfire_args(cr_batch* b, bool use_cond, cudaGraphConditionalHandle h) {
   f.fp = b->fp;
   f.st = b->status;
   f.nv = b->nv;
-  f.use_cond = use_cond ? 1 : 0;
-  f.cond = h;
   return f;
-}
-
-void enqueue_fire_iteration(cr_batch* b, cudaStream_t st, bool use_cond, cudaGraphConditionalHandle h) {
-  BFire f;
-  f.pos = b->pos;
-  f.vel = b->vel;
-  f.force = b->force;
-  f.last_pos = b->last_pos;
-  f.vsys = b->vsys;
-  f.sys_v0 = b->sys_v0_d;
-  f.bsys = b->bsys;
-  f.bfire = b->bfire;
-  f.fp = b->fp;
-  f.st = b->status;
-  f.nv = b->nv;
-  f.use_cond = use_cond ? 1 : 0;
-  f.cond = h;
-  k_bfire_pre<<<(b->nv + 255) / 256, 256, 0, st>>>(f);
-  b->launches++;
 }
 
 void enqueue_fire_tile(cr_batch* b, cudaStream_t st) {
@@ -928,32 +932,16 @@ void enqueue_fire_tile(cr_batch* b, cudaStream_t st) {
   b->launches++;
 }
 
-// n FIRE iterations onto stream st, which is capturing into graph g: each
-// iteration's rebuild is a conditional node whose body is captured on side.
-int add_fire_iterations(cr_batch* b, cudaStream_t st, cudaStream_t side, cudaGraph_t g, long n) {
+// n FIRE iterations onto stream st (capturing or not), each with the build
+// that returns at once unless the pre-kick flagged a system.
+int add_fire_iterations(cr_batch* b, cudaStream_t st, long n) {
   for (long i = 0; i < n; i++) {
-    cudaGraphConditionalHandle h = 0;
-    BT_TRY(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-    enqueue_fire_iteration(b, st, true, h);
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t cg;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    BT_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, &ndeps));
-    cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    BT_TRY(cudaGraphAddNode(&node, cg, deps, ndeps, &cp));
-    BT_TRY(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    BT_TRY(cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    enqueue_build(b, side, 0);
-    cudaGraph_t body_out;
-    BT_TRY(cudaStreamEndCapture(side, &body_out));
+    k_bfire_pre<<<(b->nv + 255) / 256, 256, 0, st>>>(bfire_args(b));
+    b->launches++;
+    enqueue_build(b, st, 0);
     enqueue_fire_tile(b, st);
   }
+  BT_TRY(cudaGetLastError());
   return CR_OK;
 }
 
@@ -971,13 +959,12 @@ BFireStepsFn persist_fn(cr_batch* b, int* block) {
   return fn;
 }
 
-// FIRE iterations with the persistent kernel onto stream st (capturing into
-// graph g): `launches` launches of up to 64 iterations, each followed by a
-// conditional rebuild (body captured on side) that runs when the launch
-// left with a system's displacement check fired, then one launch that only
-// completes a force op left pending, so the chunk ends on a whole iteration.
-int add_fire_persistent(cr_batch* b, cudaStream_t st, cudaStream_t side, cudaGraph_t g, int launches,
-                        BFireStepsFn fn, int block) {
+// FIRE iterations with the persistent kernel onto stream st (capturing or
+// not): `launches` launches of up to 64 iterations, each followed by the build
+// (at work when the launch left with a system's displacement check fired),
+// then one launch that only completes a force op left pending, so the chunk
+// ends on a whole iteration.
+int add_fire_persistent(cr_batch* b, cudaStream_t st, int launches, BFireStepsFn fn, int block) {
   StepArgs s = step_args(b);
   s.kind = KIND_FIRE;
   s.advance = 0;
@@ -986,65 +973,13 @@ int add_fire_persistent(cr_batch* b, cudaStream_t st, cudaStream_t side, cudaGra
   s.use_cond = 0;
   const SysParams p = with_f32_constants(b->p);
   for (int i = 0; i < launches; i++) {
-    cudaGraphConditionalHandle h = 0;
-    BT_TRY(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-    launch_bfire_steps(fn, tile_cfg(b, st), block, p, arrays(b), s, bfire_args(b, true, h), 64);
+    launch_bfire_steps(fn, tile_cfg(b, st), block, p, arrays(b), s, bfire_args(b), 64);
     b->launches++;
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t cg;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    BT_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, &ndeps));
-    cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    BT_TRY(cudaGraphAddNode(&node, cg, deps, ndeps, &cp));
-    BT_TRY(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    BT_TRY(cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    enqueue_build(b, side, 0);
-    cudaGraph_t body_out;
-    BT_TRY(cudaStreamEndCapture(side, &body_out));
+    enqueue_build(b, st, 0);
   }
-  launch_bfire_steps(fn, tile_cfg(b, st), block, p, arrays(b), s, bfire_args(b, false, 0), 0);
+  launch_bfire_steps(fn, tile_cfg(b, st), block, p, arrays(b), s, bfire_args(b), 0);
   b->launches++;
   BT_TRY(cudaGetLastError());
-  return CR_OK;
-}
-
-int capture_fire_persistent(cr_batch* b, BFireStepsFn fn, int block, cudaGraphExec_t* out) {
-  cudaGraph_t graph;
-  BT_TRY(cudaGraphCreate(&graph, 0));
-  BT_TRY(cudaStreamBeginCaptureToGraph(b->stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  const int rc = add_fire_persistent(b, b->stream, b->side, graph, 4, fn, block);
-  cudaGraph_t g;
-  const cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-  if (rc) {
-    cudaGraphDestroy(graph);
-    return rc;
-  }
-  BT_TRY(e);
-  BT_TRY(cudaGraphInstantiate(out, g, 0));
-  cudaGraphDestroy(g);
-  return CR_OK;
-}
-
-int capture_fire_chunk(cr_batch* b, long n, cudaGraphExec_t* out) {
-  cudaGraph_t graph;
-  BT_TRY(cudaGraphCreate(&graph, 0));
-  BT_TRY(cudaStreamBeginCaptureToGraph(b->stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  const int rc = add_fire_iterations(b, b->stream, b->side, graph, n);
-  cudaGraph_t g;
-  const cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-  if (rc) {
-    cudaGraphDestroy(graph);
-    return rc;
-  }
-  BT_TRY(e);
-  BT_TRY(cudaGraphInstantiate(out, g, 0));
-  cudaGraphDestroy(g);
   return CR_OK;
 }
 
@@ -1076,8 +1011,10 @@ int fire_prologue(cr_batch* b) {
   return CR_OK;
 }
 
-// FIRE iterations in chunks of graphs until every active system converged
-// or maxIter iterations ran.  A list overflow inside a chunk restores the
+// FIRE iterations in chunks until every active system converged or maxIter
+// iterations ran.  The launches go straight to the stream: captured chunks had to
+// be instantiated and destroyed again by every initialisation (4 ms each way for
+// 64 iterations with their conditional nodes).  A list overflow inside a chunk restores the
 // chunk's starting state, grows the lists and runs the chunk again.
 int fire_loop(cr_batch* b, long maxIter, long* done_out) {
   int rc;
@@ -1087,7 +1024,7 @@ int fire_loop(cr_batch* b, long maxIter, long* done_out) {
     if (done_out) *done_out = 0;
     return CR_OK;
   }
-  // persistent FIRE: chunks of up to 4 x 64 iterations; every system stops at
+  // persistent FIRE: chunks of up to 16 x 64 iterations; every system stops at
   // its iteration limit (fire_cap, set by the caller), so the loop ends when
   // every system has converged or reached it
   int block = 0;
@@ -1100,8 +1037,12 @@ int fire_loop(cr_batch* b, long maxIter, long* done_out) {
       return CR_OK;
     }
     if ((rc = snapshot(b, false))) return rc;
-    if (!b->pchunk && (rc = capture_fire_persistent(b, fn, block, &b->pchunk))) return rc;
-    BT_TRY(cudaGraphLaunch(b->pchunk, b->stream));
+    // launches for the iterations left, and one in case a rebuild ends one early
+    long long left = 1;
+    for (const BatchSys& s : b->bsys_h)
+      if (s.active && !s.converged) left = std::max(left, s.fire_cap - s.fire_iters);
+    const int launches = (int)std::min<long long>(16, (left + 63) / 64 + 1);
+    if ((rc = add_fire_persistent(b, b->stream, launches, fn, block))) return rc;
     if ((rc = read_status(b))) return rc;
     if (b->status_h->abort) {
       if (b->status_h->nonfinite) return b->fail(CR_ENONFINITE, "non-finite force in a batched FIRE run");
@@ -1125,15 +1066,7 @@ int fire_loop(cr_batch* b, long maxIter, long* done_out) {
     if (!any) break;
     const long n = std::min(chunk, maxIter - done);
     if ((rc = snapshot(b, false))) return rc;
-    auto key = std::make_pair(n, b->cap);
-    auto it = b->graphs.find(key);
-    if (it == b->graphs.end()) {
-      cudaGraphExec_t ge;
-      if ((rc = capture_fire_chunk(b, n, &ge))) return rc;
-      it = b->graphs.emplace(key, ge).first;
-    }
-    BT_TRY(cudaGraphLaunch(it->second, b->stream));
-    b->launches += 2 * n;
+    if ((rc = add_fire_iterations(b, b->stream, n))) return rc;
     if ((rc = read_status(b))) return rc;
     if (b->status_h->abort) {
       if (b->status_h->nonfinite) return b->fail(CR_ENONFINITE, "non-finite force in a batched FIRE run");
@@ -1251,8 +1184,8 @@ int compress_body(cr_batch* b, CompArgs a, cudaGraph_t outer_body) {
   if ((rc = add_while(b, s2, a.inner, &inner_body))) return rc;
   BT_TRY(cudaStreamBeginCaptureToGraph(s3, inner_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   int block = 0;
-  if (BFireStepsFn fn = persist_fn(b, &block)) rc = add_fire_persistent(b, s3, b->side, inner_body, 4, fn, block);
-  else rc = add_fire_iterations(b, s3, b->side, inner_body, 64);
+  if (BFireStepsFn fn = persist_fn(b, &block)) rc = add_fire_persistent(b, s3, 4, fn, block);
+  else rc = add_fire_iterations(b, s3, 64);
   if (!rc) k_cfire_more<<<1, 256, 0, s3>>>(a);
   cudaGraph_t ib_out;
   const cudaError_t e = cudaStreamEndCapture(s3, &ib_out);
@@ -1490,8 +1423,7 @@ int cr_batch_create(long numSystems, const long* numParticles, const long* nvLis
   for (int n : b->ring_nv_h)
     if (n > 128) b->block = 192;
   make_tiles(b);
-  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess) {
+  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete b;
     return CR_ECUDA;
   }
@@ -1554,7 +1486,6 @@ int cr_batch_destroy(cr_batch* b) {
     if (p) cudaFree(p);
   if (b->status_h) cudaFreeHost(b->status_h);
   if (b->stream) cudaStreamDestroy(b->stream);
-  if (b->side) cudaStreamDestroy(b->side);
   if (b->cap_s2) cudaStreamDestroy(b->cap_s2);
   if (b->cap_s3) cudaStreamDestroy(b->cap_s3);
   delete b;

@@ -22,8 +22,6 @@ struct BFire {
   FireParams fp;
   DevStatus* st;
   int nv;
-  int use_cond;
-  cudaGraphConditionalHandle cond;
 };
 
 // Vertex v: the system's FIRE scalars from its sums of the last force op

@@ -181,7 +181,8 @@ int dalloc(cr_ctx* ctx, T** p, size_t n) {
   if (n == 0) n = 1;
   cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
   if (e != cudaSuccess) return ctx->fail(CR_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  e = cudaMemset(*p, 0, n * sizeof(T));
+  // on the stream that uses the array: the default stream is not ordered with it
+  e = cudaMemsetAsync(*p, 0, n * sizeof(T), ctx->stream);
   if (e != cudaSuccess) return ctx->fail(CR_ECUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
   return CR_OK;
 }

@@ -262,8 +262,5 @@ void launch_soft_bend(cudaStream_t st, int np, const SoftArgs& a);
 void launch_soft_vertices(cudaStream_t st, int nv, const int* ring_of, const int* ring_nv, const double* a0,
                           const double* l0, const double2* ppos, const double* draws, unsigned long long seed,
                           unsigned long long stream, double2* pos, double2* vel, double2* force, double* energy);
-// building blocks shared with the batched build (cr_batch.cu)
-void launch_cell_scan(cudaStream_t st, int ncells, int* cell_cnt, int* cell_start);
-void launch_cell_sort(cudaStream_t st, int ncells, int nv, const NbrArgs& n);
 
 }  // namespace cr

@@ -676,11 +676,7 @@ __global__ void k_nbr_guard_reset(DevStatus* st) {
   }
 }
 
-void launch_cell_scan(cudaStream_t st, int ncells, int* cell_cnt, int* cell_start) {
-  k_cell_scan<<<1, 1024, 0, st>>>(ncells, cell_cnt, cell_start);
-}
-
-void launch_cell_sort(cudaStream_t st, int ncells, int nv, const NbrArgs& n) {
+static void launch_cell_sort(cudaStream_t st, int ncells, int nv, const NbrArgs& n) {
   k_cell_sort<<<(ncells + 127) / 128, 128, 0, st>>>(ncells, n.cell_start, n.cell_vid);
   k_cell_gather<<<(nv + 255) / 256, 256, 0, st>>>(nv, n.cell_start + ncells, n.cell_vid, n.pos, n.rad, n.ring_of,
                                                   n.nbr_pq ? n.pq_pack : nullptr, n.cell_pos, n.cell_rad,

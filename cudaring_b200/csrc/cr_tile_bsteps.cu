@@ -29,10 +29,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   DevStatus* st = s.status;
   const volatile DevStatus* vs = st;
   __shared__ int s_stop;
-  if (vs->abort) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && f.use_cond) cudaGraphSetConditional(f.cond, 0u);
-    return;
-  }
+  if (vs->abort) return;
   const int pending = vs->bpending;  // the last launch left with its force op due
   const int4 tile = a.tiles[blockIdx.x];
   bool stalled = false;
@@ -74,7 +71,6 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   if (stalled) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->bpending = rebuild;
-    if (f.use_cond) cudaGraphSetConditional(f.cond, (rebuild && !st->abort) ? 1u : 0u);
   }
 }
 
