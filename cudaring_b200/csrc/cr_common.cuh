@@ -241,6 +241,21 @@ struct DevStatus {
   long long spin_limit;
 };
 
+// The flags of a fresh call (counters kept).
+__host__ __device__ inline void clear_status_flags(DevStatus& s) {
+  s.abort = 0;
+  s.overflow = 0;
+  s.rebuild = 0;
+  s.converged = 0;
+  s.nonfinite = 0;
+  s.done_ctr = 0;
+  s.bar_count = 0;
+  s.stalled = 0;
+  s.pbar = 0;
+  s.pflag[0] = 0;
+  s.pbase = 0;
+}
+
 __device__ __forceinline__ long long barrier_poll_limit(const DevStatus* st) {
   const long long lim = *(const volatile long long*)&st->spin_limit;
   return lim > 0 ? lim : (lim == 0 ? (1LL << 20) : 0);

@@ -11,6 +11,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cr_copy.h"
 #include "cr_fire.cuh"
 #include "cr_launch.h"
 #include "cr_tile.cuh"
@@ -53,6 +54,7 @@ long long pow2ceil(long long x) {
 struct cr_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
+  Staging staging;
   std::string err;
   long long launches = 0;
 
@@ -161,6 +163,7 @@ struct cr_ctx {
   // state at the start of a multi-step sequence, restored if a barrier gives up
   double2 *snap_pos = nullptr, *snap_vel = nullptr, *snap_force = nullptr, *snap_last = nullptr;
   double *snap_angle = nullptr, *snap_fire = nullptr;
+  DevStatus* snap_status = nullptr;
 
   std::map<std::tuple<int, long, int, int, unsigned long long>, GraphEntry> graphs;
 
@@ -405,25 +408,24 @@ int read_status(cr_ctx* ctx) {
   return CR_OK;
 }
 
+// Flags cleared on the device; status_h is current afterwards.
 int clear_flags(cr_ctx* ctx) {
-  // abort, overflow, rebuild, converged, nonfinite <- 0 (counters kept)
   int rc = read_status(ctx);
   if (rc) return rc;
-  DevStatus s = *ctx->status_h;
-  s.abort = 0;
-  s.overflow = 0;
-  s.rebuild = 0;
-  s.converged = 0;
-  s.nonfinite = 0;
-  s.done_ctr = 0;
-  s.bar_count = 0;
-  s.stalled = 0;
-  s.pbar = 0;
-  s.pflag[0] = 0;
-  s.pbase = 0;
-  *ctx->status_h = s;
+  clear_status_flags(*ctx->status_h);
   CR_TRY(cudaMemcpyAsync(ctx->status, ctx->status_h, sizeof(DevStatus), cudaMemcpyHostToDevice, ctx->stream));
   CR_TRY(cudaStreamSynchronize(ctx->stream));
+  return CR_OK;
+}
+
+// The same without waiting; status_h is not current.
+int clear_flags_async(cr_ctx* ctx) {
+  SeqArgs a{};
+  a.st = ctx->status;
+  a.steps_left = -1;
+  launch_seq_begin(ctx->stream, a);
+  ctx->launches++;
+  CR_TRY(cudaGetLastError());
   return CR_OK;
 }
 
@@ -563,19 +565,21 @@ std::vector<Op> make_ops(cr_ctx* ctx, int kind, long nsteps) {
   return ops;
 }
 
-void enqueue_op(cr_ctx* ctx, cudaStream_t st, const Op& op, int kind, bool use_cond, cudaGraphConditionalHandle h) {
+void enqueue_op(cr_ctx* ctx, cudaStream_t st, const Op& op, int kind, bool use_cond, cudaGraphConditionalHandle h,
+                bool after_steps = false) {
   StepArgs s = base_args(ctx);
   s.kind = kind;
   s.use_cond = use_cond ? 1 : 0;
   s.cond = h;
   s.pos_out = ctx->pos[op.out_buf];
   s.advance = op.advance;
-  // per-CTA sums feed FIRE's next iteration and the rigid tail; energies
+  // per-CTA sums feed the next FIRE iteration or temperature rescale; energies
   // read by the caller are reduced afresh from the written arrays
-  s.accumulate = (kind == KIND_FIRE || kind == KIND_NVE_RESCALE || ctx->shape == CR_SHAPE_RIGID) ? 1 : 0;
+  s.accumulate = (kind == KIND_FIRE || kind == KIND_NVE_RESCALE) ? 1 : 0;
   s.rescale_T = (kind == KIND_NVE_RESCALE && op.type == OP_DRIFT) ? ctx->T : 0.0;
   s.write_out = (kind == KIND_FIRE || !op.advance) ? 1 : 0;
   s.fire_tol = ctx->fp.tol;
+  s.after_steps = after_steps ? 1 : 0;
   const SysArrays a = arrays(ctx, op.in_buf);
   const int nb = (ctx->nv + 255) / 256;
   switch (op.type) {
@@ -626,7 +630,7 @@ int capture_graph(cr_ctx* ctx, const std::vector<Op>& ops, int kind, GraphEntry&
     if (op.check_after) {
       NbrArgs nb = nbr_args(ctx, op.check_buf, ctx->cut_distance);
       nb.count_update = 1;
-      launch_nbr_fused(ctx->stream, ctx->p, ctx->grid, nb, fb, 0, ctx->shape != CR_SHAPE_RIGID);
+      launch_nbr_fused(ctx->stream, ctx->p, ctx->grid, nb, fb, 0, true);
       ge.launches++;
     }
   }
@@ -693,8 +697,9 @@ int launch_chunk(cr_ctx* ctx, const std::vector<Op>& ops, int kind, long n) {
 constexpr int kStepsPerLaunch = 64;
 constexpr int kStepsLaunches = 16;
 
-bool steps_eligible(cr_ctx* ctx, int kind, long nsteps) {
-  if (!ctx->multistep || !ctx->use_graphs || nsteps < 2) return false;
+bool steps_eligible(cr_ctx* ctx, int kind) {
+  if (!ctx->multistep || !ctx->use_graphs) return false;
+
   if (ctx->shape == CR_SHAPE_RIGID) return false;
   if (kind != KIND_NVE && kind != KIND_LANGEVIN && kind != KIND_BAOAB) return false;
   if (ctx->lanes != 1 && ctx->lanes != 2) return false;
@@ -733,27 +738,37 @@ int launch_steps(cr_ctx* ctx, int kind, int b, int launches) {
 
 int run_ops(cr_ctx* ctx, int kind, long nsteps);
 
-// The state a multi-step sequence starts from (positions, velocities,
-// forces, last-build positions, self-propulsion angles, FIRE scalars), saved or
-// restored.
-int sequence_state(cr_ctx* ctx, int b, bool restore) {
+// Start of a sequence from position buffer b: flags cleared, `steps` steps to
+// run, and the state it starts from kept (positions, velocities, forces,
+// last-build positions, self-propulsion angles, FIRE scalars, status).
+int begin_sequence(cr_ctx* ctx, int b, long long steps) {
   int rc;
   if (!ctx->snap_pos) {
     if ((rc = dalloc(ctx, &ctx->snap_pos, ctx->nv)) || (rc = dalloc(ctx, &ctx->snap_vel, ctx->nv)) ||
         (rc = dalloc(ctx, &ctx->snap_force, ctx->nv)) || (rc = dalloc(ctx, &ctx->snap_last, ctx->nv)) ||
-        (rc = dalloc(ctx, &ctx->snap_angle, ctx->np)) || (rc = dalloc(ctx, &ctx->snap_fire, 8)))
+        (rc = dalloc(ctx, &ctx->snap_angle, ctx->np)) || (rc = dalloc(ctx, &ctx->snap_fire, 8)) ||
+        (rc = dalloc(ctx, &ctx->snap_status, 1)))
       return rc;
   }
-  const size_t v2 = (size_t)ctx->nv * sizeof(double2), pa = (size_t)ctx->np * sizeof(double);
-  double2* live[4] = {ctx->pos[b], ctx->vel, ctx->force, ctx->last_pos};
-  double2* saved[4] = {ctx->snap_pos, ctx->snap_vel, ctx->snap_force, ctx->snap_last};
-  for (int k = 0; k < 4; k++)
-    CR_TRY(cudaMemcpyAsync(restore ? live[k] : saved[k], restore ? saved[k] : live[k], v2, cudaMemcpyDeviceToDevice,
-                           ctx->stream));
-  CR_TRY(cudaMemcpyAsync(restore ? ctx->p_angle : ctx->snap_angle, restore ? ctx->snap_angle : ctx->p_angle, pa,
-                         cudaMemcpyDeviceToDevice, ctx->stream));
-  CR_TRY(cudaMemcpyAsync(restore ? ctx->fire_state : ctx->snap_fire, restore ? ctx->snap_fire : ctx->fire_state,
-                         8 * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+  SeqArgs a{};
+  a.st = ctx->status;
+  a.steps_left = steps;
+  a.snap_st = ctx->snap_status;
+  const double2* from[4] = {ctx->pos[b], ctx->vel, ctx->force, ctx->last_pos};
+  double2* to[4] = {ctx->snap_pos, ctx->snap_vel, ctx->snap_force, ctx->snap_last};
+  for (int q = 0; q < 4; q++) {
+    a.from[q] = from[q];
+    a.to[q] = to[q];
+  }
+  a.angle = ctx->p_angle;
+  a.snap_angle = ctx->snap_angle;
+  a.fire = ctx->fire_state;
+  a.snap_fire = ctx->snap_fire;
+  a.nv = ctx->nv;
+  a.np = ctx->np;
+  launch_seq_begin(ctx->stream, a);
+  ctx->launches++;
+  CR_TRY(cudaGetLastError());
   return CR_OK;
 }
 
@@ -761,18 +776,22 @@ int sequence_state(cr_ctx* ctx, int b, bool restore) {
 // the sequence's positions partly advanced: go back to the state it started
 // from (counters included), rebuild the list there with the multi-kernel
 // build and run the whole sequence again one launch per op.
-int rerun_degraded(cr_ctx* ctx, int b0, const DevStatus& start, int kind, long nsteps) {
+int rerun_degraded(cr_ctx* ctx, int b0, int kind, long nsteps) {
   int rc;
   CR_TRY(cudaStreamSynchronize(ctx->stream));
-  if ((rc = sequence_state(ctx, b0, true))) return rc;
+  const size_t v2 = (size_t)ctx->nv * sizeof(double2);
+  double2* live[4] = {ctx->pos[b0], ctx->vel, ctx->force, ctx->last_pos};
+  double2* saved[4] = {ctx->snap_pos, ctx->snap_vel, ctx->snap_force, ctx->snap_last};
+  for (int k = 0; k < 4; k++)
+    CR_TRY(cudaMemcpyAsync(live[k], saved[k], v2, cudaMemcpyDeviceToDevice, ctx->stream));
+  CR_TRY(cudaMemcpyAsync(ctx->p_angle, ctx->snap_angle, (size_t)ctx->np * sizeof(double), cudaMemcpyDeviceToDevice,
+                         ctx->stream));
+  CR_TRY(cudaMemcpyAsync(ctx->fire_state, ctx->snap_fire, 8 * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+  CR_TRY(cudaMemcpyAsync(ctx->status, ctx->snap_status, sizeof(DevStatus), cudaMemcpyDeviceToDevice, ctx->stream));
   ctx->cur = b0;
-  DevStatus s = start;
-  s.abort = s.overflow = s.rebuild = s.converged = s.nonfinite = s.stalled = 0;
-  s.done_ctr = s.bar_count = s.pbar = 0;
-  s.pflag[0] = 0;
-  s.pbase = s.steps_left = 0;
-  s.bpending = 0;
-  *ctx->status_h = s;
+  if ((rc = clear_flags(ctx))) return rc;
+  ctx->status_h->steps_left = 0;
+  ctx->status_h->bpending = 0;
   if ((rc = upload(ctx, ctx->status, ctx->status_h, sizeof(DevStatus)))) return rc;
   enter_degraded(ctx);
   if ((rc = build_list(ctx, b0, ctx->cut_distance))) return rc;
@@ -783,8 +802,8 @@ int run_steps(cr_ctx* ctx, int kind, long nsteps) {
   int rc;
   int b = ctx->cur;
   const int b0 = b;
-  const DevStatus start = *ctx->status_h;  // read by the caller's clear_flags
-  if ((rc = sequence_state(ctx, b0, false))) return rc;
+  const long long middle = nsteps - 1;
+  if ((rc = begin_sequence(ctx, b0, middle))) return rc;
   // drift (first half kick + drift) and its displacement check
   enqueue_op(ctx, ctx->stream, Op{OP_DRIFT, b, b ^ 1, 0, 1, b ^ 1}, kind, false, 0);
   {
@@ -794,39 +813,38 @@ int run_steps(cr_ctx* ctx, int kind, long nsteps) {
     ctx->launches++;
   }
   b ^= 1;
-  const long long middle = nsteps - 1;
-  CR_TRY(cudaMemcpyAsync(&ctx->status->steps_left, &middle, sizeof(middle), cudaMemcpyHostToDevice, ctx->stream));
-  CR_TRY(cudaStreamSynchronize(ctx->stream));
   long long left = middle;
   for (;;) {
     const int launches =
-        (int)std::min<long long>(kStepsLaunches, std::max<long long>(2, (left + kStepsPerLaunch - 1) / kStepsPerLaunch + 1));
-    if ((rc = launch_steps(ctx, kind, b, launches))) return rc;
+        left <= 0 ? 0
+                  : (int)std::min<long long>(kStepsLaunches,
+                                             std::max<long long>(2, (left + kStepsPerLaunch - 1) / kStepsPerLaunch + 1));
+    if (launches && (rc = launch_steps(ctx, kind, b, launches))) return rc;
+    // final op: forces at the last positions and the second half kick; it
+    // does nothing while middle steps are left
+    enqueue_op(ctx, ctx->stream, Op{OP_TILE, b, b, 0, 0, b}, kind, false, 0, true);
+    CR_TRY(cudaGetLastError());
     if ((rc = read_status(ctx))) return rc;
     const DevStatus& st = *ctx->status_h;
     if (st.abort) {
-      if (st.stalled) return rerun_degraded(ctx, b0, start, kind, nsteps);
+      if (st.stalled) return rerun_degraded(ctx, b0, kind, nsteps);
       if (st.nonfinite) return ctx->fail(CR_ENONFINITE, "non-finite force during the step sequence");
       if (!st.overflow) return ctx->fail(CR_ECUDA, "step sequence aborted");
       // a rebuild found more neighbours than capacity: grow the list, rebuild
       // from the positions the failed build read (pos[b]), count the update
-      // as the in-graph build would have, and carry on
+      // as the build would have, and carry on
       if ((rc = clear_flags(ctx))) return rc;
       ctx->cap = 0;
       if ((rc = build_list(ctx, b, ctx->cut_distance))) return rc;
       if ((rc = clear_flags(ctx))) return rc;
       ctx->status_h->update_count += 1;
+      left = ctx->status_h->steps_left;
       if ((rc = upload(ctx, ctx->status, ctx->status_h, sizeof(DevStatus)))) return rc;
       continue;
     }
     if (st.steps_left <= 0) break;
     left = st.steps_left;
   }
-  // final op: forces at the last positions and the second half kick
-  enqueue_op(ctx, ctx->stream, Op{OP_TILE, b, b, 0, 0, b}, kind, false, 0);
-  CR_TRY(cudaGetLastError());
-  if ((rc = read_status(ctx))) return rc;
-  if (ctx->status_h->nonfinite) return ctx->fail(CR_ENONFINITE, "non-finite force during the step sequence");
   ctx->cur = b;
   if (ctx->status_h->max_ever > 0)
     ctx->list_size_ref = std::max<long long>(ctx->list_size_ref, pow2ceil(ctx->status_h->max_ever));
@@ -847,11 +865,7 @@ FireStepsFn fire_steps_eligible(cr_ctx* ctx, int kind) {
 int run_fire_steps(cr_ctx* ctx, FireStepsFn fn, long nsteps) {
   int rc;
   const int b = ctx->cur;
-  if ((rc = sequence_state(ctx, b, false))) return rc;
-  ctx->status_h->steps_left = nsteps;
-  ctx->status_h->bpending = 0;
-  const DevStatus start = *ctx->status_h;  // read by the caller's clear_flags
-  if ((rc = upload(ctx, ctx->status, ctx->status_h, sizeof(DevStatus)))) return rc;
+  if ((rc = begin_sequence(ctx, b, nsteps))) return rc;
   long long left = nsteps;
   for (;;) {
     StepArgs s = base_args(ctx);
@@ -876,7 +890,7 @@ int run_fire_steps(cr_ctx* ctx, FireStepsFn fn, long nsteps) {
     if ((rc = read_status(ctx))) return rc;
     const DevStatus& st = *ctx->status_h;
     if (st.abort) {
-      if (st.stalled) return rerun_degraded(ctx, b, start, KIND_FIRE, nsteps);
+      if (st.stalled) return rerun_degraded(ctx, b, KIND_FIRE, nsteps);
       if (st.nonfinite) return ctx->fail(CR_ENONFINITE, "non-finite force during the step sequence");
       if (!st.overflow) return ctx->fail(CR_ECUDA, "step sequence aborted");
       // a rebuild found more neighbours than capacity: grow the list, rebuild
@@ -920,9 +934,9 @@ int run_ops(cr_ctx* ctx, int kind, long nsteps) {
     ctx->launches++;
     CR_TRY(cudaGetLastError());
   }
-  if ((rc = clear_flags(ctx))) return rc;
-  if (steps_eligible(ctx, kind, nsteps)) return run_steps(ctx, kind, nsteps);
+  if (steps_eligible(ctx, kind)) return run_steps(ctx, kind, nsteps);
   if (FireStepsFn fn = fire_steps_eligible(ctx, kind)) return run_fire_steps(ctx, fn, nsteps);
+  if ((rc = clear_flags(ctx))) return rc;
   const long chunk = 128;
   std::vector<std::vector<Op>> plan;
   std::vector<long> sizes;
@@ -1010,16 +1024,14 @@ int set_current_device(cr_ctx* ctx) {
 
 int upload(cr_ctx* ctx, void* dst, const void* src, size_t bytes) {
   if (!src) return ctx->fail(CR_EINVAL, "NULL host pointer");
-  CR_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
-  CR_TRY(cudaStreamSynchronize(ctx->stream));
+  CR_TRY(copy_in(ctx->staging, ctx->device, ctx->stream, dst, src, bytes));
   return CR_OK;
 }
 
 int download(const cr_ctx* cctx, void* dst, const void* src, size_t bytes) {
   cr_ctx* ctx = const_cast<cr_ctx*>(cctx);
   if (!dst) return ctx->fail(CR_EINVAL, "NULL host pointer");
-  CR_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-  CR_TRY(cudaStreamSynchronize(ctx->stream));
+  CR_TRY(copy_out(ctx->staging, ctx->device, ctx->stream, dst, src, bytes));
   return CR_OK;
 }
 
@@ -1168,7 +1180,7 @@ int cr_destroy(cr_ctx* ctx) {
                   ctx->p_torque, ctx->p_moi, ctx->v_torque, ctx->sp_angle, ctx->block_sum, ctx->cell_bucket, ctx->bucket_pos, ctx->bucket_rad,
                   ctx->bucket_ring, ctx->bucket_pq,
                   ctx->prad, ctx->plast, ctx->pid, ctx->pnbr, ctx->pnbr_cnt, ctx->pstatus, ctx->pfire, ctx->pdraws,
-                  ctx->snap_pos, ctx->snap_vel, ctx->snap_force, ctx->snap_last, ctx->snap_angle, ctx->snap_fire};
+                  ctx->snap_pos, ctx->snap_vel, ctx->snap_force, ctx->snap_last, ctx->snap_angle, ctx->snap_fire, ctx->snap_status};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (ctx->status_h) cudaFreeHost(ctx->status_h);
@@ -1452,7 +1464,7 @@ int cr_set_displacement_cutoff(cr_ctx* ctx, double cutoff, double size, double* 
 
 int cr_calc_neighbor_list(cr_ctx* ctx, double cut) {
   if (!ctx) return CR_EINVAL;
-  int rc = clear_flags(ctx);
+  int rc = clear_flags_async(ctx);
   if (rc) return rc;
   return build_list(ctx, ctx->cur, cut);
 }
@@ -1792,7 +1804,7 @@ static int fire_run(cr_ctx* ctx, long nsteps, double tol) {
   ctx->fp.tol = tol;
   drop_graphs(ctx);
   if ((rc = reduce_now(ctx))) return rc;  // P, |v|^2, |F|^2 of the current state
-  if ((rc = clear_flags(ctx))) return rc;
+  if ((rc = clear_flags_async(ctx))) return rc;
   if (tol >= 0 && ctx->status_h->sums[S_FMAX2] <= tol * tol) return CR_OK;
   return run_ops(ctx, KIND_FIRE, nsteps);
 }

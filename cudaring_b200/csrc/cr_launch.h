@@ -47,6 +47,21 @@ struct FireParams {
   long long min_step;
   double tol;
 };
+// Start of a sequence: flags cleared (and, with steps_left >= 0, the count of
+// steps to run set); with snap_st the state it starts from is kept.
+struct SeqArgs {
+  DevStatus* st;
+  long long steps_left;
+  DevStatus* snap_st;   // nullable: nothing is kept
+  const double2* from[4];
+  double2* to[4];       // nv each
+  const double* angle;
+  double* snap_angle;   // np
+  const double* fire;
+  double* snap_fire;    // 8
+  int nv, np;
+};
+void launch_seq_begin(cudaStream_t st, const SeqArgs& a);
 void launch_drift(cudaStream_t st, const SysParams& p, const SysArrays& a, const StepArgs& s, int nblocks);
 void launch_fire_pre(cudaStream_t st, const SysParams& p, const SysArrays& a, const StepArgs& s,
                      const FireParams& fp, double* fire_state, int nblocks);

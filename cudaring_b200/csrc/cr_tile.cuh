@@ -76,6 +76,7 @@ struct StepArgs {
   const double* bfire_state;  // batch mode: [S][2][4] FIRE scalars per system
   unsigned long long seed;
   int persist_max;          // multi-step kernel: most steps per launch
+  int after_steps;          // the op runs only once no middle step is left (the last op of a sequence)
 };
 
 // ------------------------------------------------------------------ helpers

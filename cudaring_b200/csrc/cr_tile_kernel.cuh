@@ -1440,7 +1440,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
   pdl_wait();
   pdl_trigger();
   DevStatus* st = s.status;
-  if (MODE == MODE_STEP && (st->abort | st->converged)) {
+  if (MODE == MODE_STEP && ((st->abort | st->converged) || (s.after_steps && st->steps_left > 0))) {
     // keep the last-block protocol intact so later ops see a consistent counter
     if (is_last_block(st)) {
       if (threadIdx.x == 0) {

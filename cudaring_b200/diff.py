@@ -61,12 +61,19 @@ def _energy(d: DPM2D) -> float:
     return d.getPotentialEnergy() + d.getKineticEnergy()
 
 
-def _refresh(d: DPM2D, x: np.ndarray, v: np.ndarray | None = None) -> None:
+def _refresh(d: DPM2D, x: np.ndarray, v: np.ndarray | None = None, cut: float | None = None,
+             forces: bool = True) -> float:
+    """Positions (and velocities) with a fresh list and, if asked for, forces;
+    returns the list's cut distance (from the vertex radii unless given)."""
     d.setVertexPositions(x)
     if v is not None:
         d.setVertexVelocities(v)
-    d.calcNeighborList(d.setDisplacementCutoff(0.5, 2.0 * d.getMeanVertexRadius()))
-    d.calcForceEnergy()
+    if cut is None:
+        cut = d.setDisplacementCutoff(0.5, 2.0 * d.getMeanVertexRadius())
+    d.calcNeighborList(cut)
+    if forces:
+        d.calcForceEnergy()
+    return cut
 
 
 def nve_run(d: DPM2D, x0: np.ndarray, v0: np.ndarray, nsteps: int, dt: float) -> float:
@@ -82,7 +89,7 @@ def nve_gradient(d: DPM2D, x0: np.ndarray, v0: np.ndarray, nsteps: int, dt: floa
     """(J, dJ/dx0, dJ/dv0) with checkpoints every ``checkpoint`` steps."""
     d.setTimeStep(dt)
     h = dt
-    _refresh(d, x0, v0)
+    cut = _refresh(d, x0, v0)
     d.initNVE(0.0, readState=True)
     cps = [(x0.copy(), v0.copy())]
     done = 0
@@ -93,7 +100,7 @@ def nve_gradient(d: DPM2D, x0: np.ndarray, v0: np.ndarray, nsteps: int, dt: floa
         cps.append((d.getVertexPositions(), d.getVertexVelocities()))
     J = _energy(d)
     xN, vN = cps[-1]
-    _refresh(d, xN)
+    _refresh(d, xN, cut=cut)
     xb = -d.getVertexForces()
     vb = vN.copy()
     seg_starts = list(range(0, nsteps, checkpoint))
@@ -102,15 +109,18 @@ def nve_gradient(d: DPM2D, x0: np.ndarray, v0: np.ndarray, nsteps: int, dt: floa
         n1 = min(n0 + checkpoint, nsteps)
         # recompute the segment's positions x_n0 .. x_n1
         xs = [cps[k][0]]
-        _refresh(d, cps[k][0], cps[k][1])
+        _refresh(d, cps[k][0], cps[k][1], cut)
         d.initNVE(0.0, readState=True)
         for _ in range(n1 - n0):
             d.NVELoop(1)
             xs.append(d.getVertexPositions())
+        # products at x_{m+1}, then at x_m, where the next step's first one is
+        # taken too: each position is set once; the forces are those of the
+        # last one only
+        _refresh(d, xs[n1 - n0], cut=cut, forces=False)
         for m in reversed(range(n1 - n0)):
-            _refresh(d, xs[m + 1])
             xb = xb - 0.5 * h * d.hvp(vb)
             vb = vb + h * xb
-            _refresh(d, xs[m])
+            _refresh(d, xs[m], cut=cut, forces=m == 0)
             xb = xb - 0.5 * h * d.hvp(vb)
     return J, xb, vb
