@@ -24,26 +24,52 @@
 
 namespace cr {
 
+// Sums of N arrays over v[f .. f + n) by one warp, left in v[f].
+template <int N>
+__device__ __forceinline__ void ring_sums(double* const (&v)[N], int f, int n) {
+  const int wl = threadIdx.x & 31;
+  double x[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) x[q] = 0.0;
+  for (int c = wl; c < n; c += 32)
+#pragma unroll
+    for (int q = 0; q < N; q++) x[q] += v[q][f + c];
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < N; q++) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
+  if (wl == 0)
+#pragma unroll
+    for (int q = 0; q < N; q++) v[q][f] = x[q];
+}
+
 // PREC_MIXED: the vertex pair terms in FP32 on FP64-formed offsets (as the
 // deformable kernel's mixed path), accumulated per vertex in FP32; torques,
 // ring sums and integration stay FP64.
+//
+// A step is a chain of short phases, bound by latency: the ring sums take one
+// warp per ring (a tree over shared memory took a CTA barrier per level, twice
+// seven of them), the rings' random numbers are drawn before the pair phase,
+// the rotation's sine and cosine once per ring, and no sums over the system
+// are formed (nothing reads them).  100 steps with 4 or 5 rebuilds, one graph
+// captured for them: 98,304 vertices, WCA, FP64, 4.10 -> 2.82 ms; 36,024
+// vertices, FP32 pairs, 2.41 -> 1.97 ms.
 template <int POT, int MODE, int BLOCK, int L, int PREC>
 __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysParams p,
                                                  const __grid_constant__ SysArrays a,
                                                  const __grid_constant__ StepArgs s,
                                                  const __grid_constant__ RigidArgs r) {
-  constexpr int TV = BLOCK / L;
+  constexpr int TV = BLOCK / L, W = BLOCK / 32;
   __shared__ double2 s_pos[TV];
-  __shared__ double2 s_u[TV];     // offsets from the ring's first vertex -> centroid
-  __shared__ double2 s_f[TV];     // pair force
+  __shared__ double s_ux[TV], s_uy[TV];   // offsets from the ring's first vertex -> centroid
+  __shared__ double2 s_f[TV];             // pair force
   __shared__ double s_e[TV];
-  __shared__ double2 s_rf[TV];    // ring sums
-  __shared__ double s_rt[TV], s_rm[TV], s_re[TV];
-  __shared__ double2 s_c[TV];     // centroid per vertex slot (valid at the ring's first vertex)
-  __shared__ double2 s_shift[TV]; // ring translation for this op (first vertex slot)
-  __shared__ double s_dang[TV];   // ring rotation for this op (first vertex slot)
-  __shared__ double s_red[BLOCK / 32][NSUM];
+  __shared__ double s_rx[TV], s_ry[TV], s_rt[TV], s_rm[TV], s_re[TV];  // ring sums (at the first vertex)
+  __shared__ int s_first[TV], s_len[TV];  // per ring of the tile: first vertex, vertices
+  __shared__ double2 s_c[TV], s_shift[TV], s_rot[TV], s_noise[TV];  // per ring: centroid, translation, rotation, draws
+  __shared__ double s_draw[TV];
 
+  pdl_wait();
+  pdl_trigger();
   DevStatus* st = s.status;
   if (MODE == MODE_STEP && (st->abort | st->converged)) {
     if (is_last_block(st)) {
@@ -56,46 +82,77 @@ __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysPara
   }
   const int4 tile = a.tiles[blockIdx.x];
   const int v0 = tile.z, nvt = tile.w - tile.z;
-  const int t = threadIdx.x;
-  int ring = -1, k = 0, lf = 0, nvr = 1;
+  const int ring0 = tile.x, nrings = tile.y - tile.x;
+  const int t = threadIdx.x, w = t / 32;
+  const int lv = t / L, lane = t % L;
+  const unsigned long long step = MODE == MODE_STEP ? (unsigned long long)st->rng_step : 0ull;
+  int q0 = 0, lf = 0, k = 0, nvr = 1;  // ring in the tile, its first vertex
   if (t < nvt) {
-    const int v = v0 + t;
-    ring = a.ring_of[v];
-    nvr = a.ring_nv[ring];
-    lf = a.ring_first[ring] - v0;
-    k = t - lf;
-    s_pos[t] = a.pos[v];
-  }
-  __syncthreads();
-  if (t < nvt) s_u[t] = pbc2(p, s_pos[t], s_pos[lf]);
-  for (int stride = 1; stride < TV; stride <<= 1) {
-    __syncthreads();
-    if (t < nvt && (k % (2 * stride)) == 0 && k + stride < nvr) {
-      s_u[t].x += s_u[t + stride].x;
-      s_u[t].y += s_u[t + stride].y;
+    const int2 tp = __ldg(a.vtopo + v0 + t);
+    q0 = tp.x - ring0;
+    k = tp.y & 0xffff;
+    nvr = tp.y >> 16;
+    lf = t - k;
+    s_pos[t] = __ldg(a.pos + v0 + t);
+    if (k == 0) {
+      s_first[q0] = t;
+      s_len[q0] = nvr;
     }
   }
+  // list counts and first slots, in flight across the centroid phase
+  int cnt = 0, j1 = 0, j2 = 0;
+  double ri = 0.0;
+  if (lv < nvt) {
+    cnt = min(__ldg(a.nbr_cnt + v0 + lv), a.nbr_cap);
+    ri = __ldg(a.rad + v0 + lv);
+    if (lane < cnt) j1 = __ldg(a.nbr + (size_t)lane * p.nv + v0 + lv);
+    if (lane + L < cnt) j2 = __ldg(a.nbr + (size_t)(lane + L) * p.nv + v0 + lv);
+  }
+  if (MODE == MODE_STEP && BLOCK - 1 - t < nrings) {
+    // the rings' random numbers, by the last threads (with two or more lanes
+    // these have no vertex in the phases before the pairs)
+    const int q = BLOCK - 1 - t;
+    const unsigned long long ring = (unsigned long long)(ring0 + q);
+    if (s.kind == KIND_LANGEVIN) s_noise[q] = philox_normal2(s.seed, 2ull * step, ring);
+    if (s.active) s_draw[q] = philox_normal2(s.seed, 2ull * step + 1ull, ring).x;
+  }
   __syncthreads();
-  if (t < nvt && k == 0) {
-    const double2 x0 = s_pos[t];
-    s_c[t] = make_double2(x0.x + s_u[t].x / nvr, x0.y + s_u[t].y / nvr);
+  if (t < nvt) {
+    const double2 u = pbc2(p, s_pos[t], s_pos[lf]);
+    s_ux[t] = u.x;
+    s_uy[t] = u.y;
+  }
+  __syncthreads();
+  for (int q = w; q < nrings; q += W) {
+    double* const arr[2] = {s_ux, s_uy};
+    const int f = s_first[q], n = s_len[q];
+    ring_sums<2>(arr, f, n);
+    if ((t & 31) == 0) s_c[q] = make_double2(s_pos[f].x + s_ux[f] / n, s_pos[f].y + s_uy[f] / n);
   }
 
-  // pair forces
+  // pair forces: the next slot's neighbour is fetched before this one's term
   {
-    const int lv = t / L, lane = t % L;
     using T = typename std::conditional<PREC == PREC_MIXED, float, double>::type;
     typename Vec2<T>::type fi{0, 0};
     double ei = 0.0;
     if (lv < nvt) {
-      const int i = v0 + lv;
       const double2 xi = s_pos[lv];
-      const double ri = a.rad[i];
-      const int cnt = min(a.nbr_cnt[i], a.nbr_cap);
+      double2 nx = make_double2(0.0, 0.0);
+      double nr = 0.0;
+      if (lane < cnt) {
+        nx = __ldg(a.pos + j1);
+        nr = __ldg(a.rad + j1);
+      }
       for (int sl = lane; sl < cnt; sl += L) {
-        const int j = __ldg(a.nbr + (size_t)sl * p.nv + i);
-        if constexpr (PREC == PREC_MIXED) pair_own_f<POT>(p, f2(pbc2(p, xi, a.pos[j])), (float)(ri + __ldg(a.rad + j)), fi, ei);
-        else pair_own<POT>(p, pbc2(p, xi, a.pos[j]), ri + __ldg(a.rad + j), fi, ei);
+        const double2 xj = nx;
+        const double rj = nr;
+        if (sl + L < cnt) {
+          nx = __ldg(a.pos + j2);
+          nr = __ldg(a.rad + j2);
+          if (sl + 2 * L < cnt) j2 = __ldg(a.nbr + (size_t)(sl + 2 * L) * p.nv + v0 + lv);
+        }
+        if constexpr (PREC == PREC_MIXED) pair_own_f<POT>(p, f2(pbc2(p, xi, xj)), (float)(ri + rj), fi, ei);
+        else pair_own<POT>(p, pbc2(p, xi, xj), ri + rj, fi, ei);
       }
     }
 #pragma unroll
@@ -112,38 +169,34 @@ __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysPara
   __syncthreads();
 
   // torque about the centroid and ring sums
-  double2 F = make_double2(0.0, 0.0), rel = make_double2(0.0, 0.0);
+  double2 F = make_double2(0.0, 0.0);
   double tau = 0.0;
   if (t < nvt) {
     F = s_f[t];
-    rel = pbc2(p, s_pos[t], s_c[lf]);
+    const double2 rel = pbc2(p, s_pos[t], s_c[q0]);
     tau = rel.x * F.y - rel.y * F.x;
-    s_rf[t] = F;
+    s_rx[t] = F.x;
+    s_ry[t] = F.y;
     s_rt[t] = tau;
     s_rm[t] = rel.x * rel.x + rel.y * rel.y;
     s_re[t] = s_e[t];
   }
-  for (int stride = 1; stride < TV; stride <<= 1) {
-    __syncthreads();
-    if (t < nvt && (k % (2 * stride)) == 0 && k + stride < nvr) {
-      s_rf[t].x += s_rf[t + stride].x;
-      s_rf[t].y += s_rf[t + stride].y;
-      s_rt[t] += s_rt[t + stride];
-      s_rm[t] += s_rm[t + stride];
-      s_re[t] += s_re[t + stride];
-    }
+  __syncthreads();
+  for (int q = w; q < nrings; q += W) {
+    double* const arr[5] = {s_rx, s_ry, s_rt, s_rm, s_re};
+    ring_sums<5>(arr, s_first[q], s_len[q]);
   }
   __syncthreads();
 
   if constexpr (MODE == MODE_FORCE) {
     if (t < nvt) {
-      const int v = v0 + t;
+      const int v = v0 + t, ring = ring0 + q0;
       s.force[v] = F;
       s.energy[v] = s_e[t];
       r.v_torque[v] = tau;
       if (k == 0) {
-        s.ppos_out[ring] = s_c[t];
-        r.p_force[ring] = s_rf[t];
+        s.ppos_out[ring] = s_c[q0];
+        r.p_force[ring] = make_double2(s_rx[t], s_ry[t]);
         r.p_torque[ring] = s_rt[t] / s_rm[t];
         r.p_moi[ring] = s_rm[t];
         s.p_energy[ring] = s_re[t];
@@ -151,16 +204,16 @@ __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysPara
     }
     return;
   } else {
-    double sums[NSUM] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const unsigned long long step = (unsigned long long)st->rng_step;
-    if (t < nvt && k == 0) {
-      double2 Fp = s_rf[t];
-      const double alpha = s_rt[t] / s_rm[t];
+    int nonfinite = 0;
+    if (t < nrings) {
+      // ring t of the tile
+      const int ring = ring0 + t, f = s_first[t];
+      double2 Fp = make_double2(s_rx[f], s_ry[f]);
+      const double alpha = s_rt[f] / s_rm[f];
       if (s.active) {
         // self-propulsion of the ring along its own diffusing angle
         double psi = r.sp_angle[ring];
-        const double2 z = philox_normal2(s.seed, 2ull * step + 1ull, (unsigned long long)ring);
-        psi += s.sp_amp * z.x;
+        psi += s.sp_amp * s_draw[t];
         psi = psi + kPi;
         psi = psi - 2.0 * kPi * floor(psi / (2.0 * kPi));
         psi = psi - kPi;
@@ -173,7 +226,7 @@ __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysPara
       const double2 vh = r.p_vel[ring];
       const double wh = r.p_angvel[ring];
       if (s.kind == KIND_LANGEVIN) {
-        const double2 z = philox_normal2(s.seed, 2ull * step, (unsigned long long)ring);
+        const double2 z = s_noise[t];
         Fp.x += s.noise * z.x - s.gamma * vh.x;
         Fp.y += s.noise * z.y - s.gamma * vh.y;
       }
@@ -186,39 +239,31 @@ __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysPara
         r.p_angvel[ring] = w2;
         r.p_angle[ring] += s.dt * w2;
         s_shift[t] = make_double2(s.dt * v2.x, s.dt * v2.y);
-        s_dang[t] = s.dt * w2;
+        double sn, cs;
+        sincos(s.dt * w2, &sn, &cs);
+        s_rot[t] = make_double2(cs, sn);
       } else {
         r.p_vel[ring] = vn;
         r.p_angvel[ring] = wn;
         r.p_force[ring] = Fp;
         r.p_torque[ring] = alpha;
-        r.p_moi[ring] = s_rm[t];
-        s.p_energy[ring] = s_re[t];
+        r.p_moi[ring] = s_rm[f];
+        s.p_energy[ring] = s_re[f];
         s.ppos_out[ring] = s_c[t];
       }
-      if (s.accumulate) {
-        sums[S_PE] = s_re[t];
-        sums[S_VV] = vn.x * vn.x + vn.y * vn.y;
-        sums[S_VF] = vn.x * Fp.x + vn.y * Fp.y;
-        sums[S_FF] = Fp.x * Fp.x + Fp.y * Fp.y;
-        sums[S_FMAX2] = fmax(Fp.x * Fp.x, Fp.y * Fp.y);
-      }
-      if (!(isfinite(Fp.x) && isfinite(Fp.y) && isfinite(alpha))) sums[S_NONFINITE] = 1.0;
+      nonfinite = !(isfinite(Fp.x) && isfinite(Fp.y) && isfinite(alpha));
     }
-    __syncthreads();
+    const bool bad = __syncthreads_or(nonfinite) != 0;
     if (t < nvt) {
       const int v = v0 + t;
       if (s.advance) {
         // kernelTranslateVertices then kernelRotateVertices about the new centroid
-        const double2 sh = s_shift[lf];
-        const double da = s_dang[lf];
-        const double2 cn = make_double2(s_c[lf].x + sh.x, s_c[lf].y + sh.y);
+        const double2 sh = s_shift[q0], rot = s_rot[q0];
+        const double2 cn = make_double2(s_c[q0].x + sh.x, s_c[q0].y + sh.y);
         double2 x = make_double2(s_pos[t].x + sh.x, s_pos[t].y + sh.y);
         const double2 d = pbc2(p, x, cn);
-        double sn, cs;
-        sincos(da, &sn, &cs);
-        x.x += (d.x * cs - d.y * sn) - d.x;
-        x.y += (d.x * sn + d.y * cs) - d.y;
+        x.x += (d.x * rot.x - d.y * rot.y) - d.x;
+        x.y += (d.x * rot.y + d.y * rot.x) - d.y;
         s.pos_out[v] = x;
         if (3.0 * dist_of(pbc2(p, x, s.last_pos[v])) > s.disp_cutoff) st->rebuild = 1;
       } else {
@@ -227,16 +272,13 @@ __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysPara
         r.v_torque[v] = tau;
       }
     }
-    block_partials<BLOCK>(sums, s_red, s.partials + (size_t)blockIdx.x * NSUM);
+    if (bad && t == 0) {
+      st->nonfinite = 1;
+      st->abort = 1;
+    }
     if (is_last_block(st)) {
-      reduce_partials(s.partials, gridDim.x, st->sums);
-      __syncthreads();
       if (t == 0) {
         __threadfence();
-        if (st->sums[S_NONFINITE] != 0.0) {
-          st->nonfinite = 1;
-          st->abort = 1;
-        }
         st->ops_done += 1;
         st->rng_step += 1;
         st->done_ctr = 0;
@@ -343,10 +385,10 @@ __global__ void k_rigid_inject(int np, double2* p_vel, double amp, unsigned long
 template <int POT, int MODE, int PREC>
 static void launch_rigid_p(const LaunchCfg& c, const SysParams& p, const SysArrays& a, const StepArgs& s,
                            const RigidArgs& r) {
-  if (c.lanes == 1) k_rigid<POT, MODE, 128, 1, PREC><<<c.grid, 128, 0, c.stream>>>(p, a, s, r);
-  else if (c.lanes == 4) k_rigid<POT, MODE, 256, 4, PREC><<<c.grid, 256, 0, c.stream>>>(p, a, s, r);
-  else if (c.lanes == 8) k_rigid<POT, MODE, 256, 8, PREC><<<c.grid, 256, 0, c.stream>>>(p, a, s, r);
-  else k_rigid<POT, MODE, 192, 2, PREC><<<c.grid, 192, 0, c.stream>>>(p, a, s, r);  // tiles of up to 96 vertices
+  if (c.lanes == 1) launch_k(c.pdl, k_rigid<POT, MODE, 128, 1, PREC>, dim3(c.grid), dim3(128), c.stream, 0, p, a, s, r);
+  else if (c.lanes == 4) launch_k(c.pdl, k_rigid<POT, MODE, 256, 4, PREC>, dim3(c.grid), dim3(256), c.stream, 0, p, a, s, r);
+  else if (c.lanes == 8) launch_k(c.pdl, k_rigid<POT, MODE, 256, 8, PREC>, dim3(c.grid), dim3(256), c.stream, 0, p, a, s, r);
+  else launch_k(c.pdl, k_rigid<POT, MODE, 192, 2, PREC>, dim3(c.grid), dim3(192), c.stream, 0, p, a, s, r);  // tiles of up to 96 vertices
 }
 
 template <int POT, int MODE>
