@@ -616,24 +616,30 @@ void enqueue_op(cr_ctx* ctx, cudaStream_t st, const Op& op, int kind, bool use_c
   ctx->launches++;
 }
 
-// A step sequence as one graph.  Every op that may arm a rebuild (its
+// A step sequence onto the stream.  Every op that may arm a rebuild (its
 // displacement check) is followed by the one-launch build, which returns at
 // once unless the check fired (DPM2D::checkDisplacement, src/DPM2D.cu:1397-1405,
 // rebuilds and counts an update).
-int capture_graph(cr_ctx* ctx, const std::vector<Op>& ops, int kind, GraphEntry& ge) {
-  CR_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+long long enqueue_chunk(cr_ctx* ctx, const std::vector<Op>& ops, int kind) {
   const int fb = nbr_fused_blocks(ctx->nv, ctx->fused_max);
-  ge.launches = 0;
+  long long launches = 0;
   for (const Op& op : ops) {
     enqueue_op(ctx, ctx->stream, op, kind, false, 0);
-    ge.launches++;
+    launches++;
     if (op.check_after) {
       NbrArgs nb = nbr_args(ctx, op.check_buf, ctx->cut_distance);
       nb.count_update = 1;
       launch_nbr_fused(ctx->stream, ctx->p, ctx->grid, nb, fb, 0, true);
-      ge.launches++;
+      launches++;
     }
   }
+  return launches;
+}
+
+// The same as one graph.
+int capture_graph(cr_ctx* ctx, const std::vector<Op>& ops, int kind, GraphEntry& ge) {
+  CR_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+  ge.launches = enqueue_chunk(ctx, ops, kind);
   cudaGraph_t out = nullptr;
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &out);
   if (e != cudaSuccess) {
@@ -664,7 +670,18 @@ int run_direct(cr_ctx* ctx, const std::vector<Op>& ops, size_t first, int kind) 
   return CR_OK;
 }
 
-int launch_chunk(cr_ctx* ctx, const std::vector<Op>& ops, int kind, long n) {
+// chunks: how many chunks the call runs.  A graph pays once several of them
+// replay it: capturing, instantiating and destroying one costs some 4 us per op
+// (0.5 ms for 100 rigid steps, whose kernels take 1.5), a plain launch 2 us, less
+// than the op takes.
+constexpr size_t kGraphChunks = 8;
+int launch_chunk(cr_ctx* ctx, const std::vector<Op>& ops, int kind, long n, size_t chunks) {
+  if (ctx->use_graphs && chunks < kGraphChunks) {
+    const long long before = ctx->launches;
+    ctx->launches = before + enqueue_chunk(ctx, ops, kind);
+    CR_TRY(cudaGetLastError());
+    return CR_OK;
+  }
   if (ctx->use_graphs) {
     auto key = std::make_tuple(kind, n, ops.front().in_buf, ctx->cap, 0ULL);
     auto it = ctx->graphs.find(key);
@@ -958,11 +975,11 @@ int run_ops(cr_ctx* ctx, int kind, long nsteps) {
     const long long ops0 = ctx->status_h->ops_done;
     size_t c_end = c;
     if (kind == KIND_FIRE) {
-      if ((rc = launch_chunk(ctx, plan[c], kind, sizes[c]))) return rc;
+      if ((rc = launch_chunk(ctx, plan[c], kind, sizes[c], plan.size()))) return rc;
       c_end = c + 1;
     } else {
       for (c_end = c; c_end < plan.size(); c_end++)
-        if ((rc = launch_chunk(ctx, plan[c_end], kind, sizes[c_end]))) return rc;
+        if ((rc = launch_chunk(ctx, plan[c_end], kind, sizes[c_end], plan.size()))) return rc;
     }
     if ((rc = read_status(ctx))) return rc;
     if (ctx->status_h->abort) {
