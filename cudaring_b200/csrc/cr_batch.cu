@@ -97,7 +97,7 @@ struct cr_batch {
   cudaStream_t cap_s2 = nullptr, cap_s3 = nullptr;  // capture streams of the nested loop bodies
   cudaGraphExec_t comp_exec = nullptr;
   // persistent batched FIRE (k_bfire_steps): off by request or after a
-  // grid-barrier wait gave up; the chunk graph of the current list capacity
+  // grid-barrier wait gave up
   bool no_persist = false;
   std::map<BFireStepsFn, int> persist_max;  // CTAs each kernel holds resident at once
   long long launches = 0;
@@ -447,8 +447,7 @@ __global__ void k_bsave(int nv, int np, const int* vsys, const int* ring_sys, co
 //
 // The compressFIRE protocol of cr_batch_compress as one CUDA graph: an outer
 // WHILE node over compression steps and, inside it, a WHILE node over chunks
-// of FIRE iterations (the chunk of the host loop, with its conditional
-// rebuild nodes).  Every decision the host loop makes between launches is
+// of FIRE iterations (the chunk of the host loop).  Every decision the host loop makes between launches is
 // made here by a kernel, with the host loop's arithmetic in the host loop's
 // order (per-system sums run sequentially on one thread), so both loops
 // produce the same states.
@@ -904,8 +903,8 @@ int reduce_sys(cr_batch* b, int set_converged, cudaStream_t st = nullptr) {
 }
 
 // One FIRE iteration over every unconverged system: pre-kick (with the
-// displacement check), conditional rebuild of the flagged systems, force +
-// second kick with per-system sums and convergence.
+// displacement check), the build of the flagged systems, force + second kick
+// with per-system sums and convergence.
 BFire bfire_args(cr_batch* b) {
   BFire f;
   f.pos = b->pos;
@@ -1014,8 +1013,8 @@ int fire_prologue(cr_batch* b) {
 // FIRE iterations in chunks until every active system converged or maxIter
 // iterations ran.  The launches go straight to the stream: captured chunks had to
 // be instantiated and destroyed again by every initialisation (4 ms each way for
-// 64 iterations with their conditional nodes).  A list overflow inside a chunk restores the
-// chunk's starting state, grows the lists and runs the chunk again.
+// 64 iterations).  A list overflow inside a chunk restores the chunk's starting
+// state, grows the lists and runs the chunk again.
 int fire_loop(cr_batch* b, long maxIter, long* done_out) {
   int rc;
   long done = 0;

@@ -1,6 +1,8 @@
-// Context, op sequencer (CUDA graphs of step ops, each followed by the
-// one-launch neighbour build that runs only when the op armed it) and the
-// C ABI declared in include/cudaring.h.
+// Context, op sequencer (step ops, each followed by the one-launch neighbour
+// build that runs only when the op armed it, launched one by one or, in calls
+// of many chunks, as a captured graph; sequences of steps and of FIRE
+// iterations in multi-step kernels) and the C ABI declared in
+// include/cudaring.h.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -2260,8 +2262,8 @@ extern "C" int cr_param_derivatives(cr_ctx* ctx, int param, double* dU, double* 
 }
 
 // Scratch and tiles of k_cg_steps; *ok = false where it does not apply (smooth
-// interaction, a grid the GPU does not hold at once, a barrier that gave up
-// before).
+// interaction, a grid the GPU does not hold at once, no memory for the rows, a
+// barrier that gave up before).
 static int cg_steps_ready(cr_ctx* ctx, bool* ok) {
   *ok = false;
   if (!ctx->cg_steps || ctx->degraded || inter_kind(ctx) != INT_VV) return CR_OK;
@@ -2301,9 +2303,11 @@ static int cg_steps_ready(cr_ctx* ctx, bool* ok) {
   if (cg_steps_max_blocks(ctx->potential, ctx->cgs_block) < ctx->cgs_ntiles) return CR_OK;
   if (ctx->cgs_cap < ctx->cap) {
     const size_t n = (size_t)ctx->cap * ctx->nv;
-    if ((rc = dalloc(ctx, &ctx->cgs_kxy, n)) || (rc = dalloc(ctx, &ctx->cgs_kyy, n)) ||
-        (rc = dalloc(ctx, &ctx->cgs_kj, n)))
-      return rc;
+    if (dalloc(ctx, &ctx->cgs_kxy, n) || dalloc(ctx, &ctx->cgs_kyy, n) || dalloc(ctx, &ctx->cgs_kj, n)) {
+      cudaGetLastError();  // no room for the rows: one launch per op needs none
+      ctx->cg_steps = false;
+      return CR_OK;
+    }
     ctx->cgs_cap = ctx->cap;
   }
   *ok = true;

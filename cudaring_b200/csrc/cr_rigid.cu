@@ -24,24 +24,6 @@
 
 namespace cr {
 
-// Sums of N arrays over v[f .. f + n) by one warp, left in v[f].
-template <int N>
-__device__ __forceinline__ void ring_sums(double* const (&v)[N], int f, int n) {
-  const int wl = threadIdx.x & 31;
-  double x[N];
-#pragma unroll
-  for (int q = 0; q < N; q++) x[q] = 0.0;
-  for (int c = wl; c < n; c += 32)
-#pragma unroll
-    for (int q = 0; q < N; q++) x[q] += v[q][f + c];
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int q = 0; q < N; q++) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
-  if (wl == 0)
-#pragma unroll
-    for (int q = 0; q < N; q++) v[q][f] = x[q];
-}
-
 // PREC_MIXED: the vertex pair terms in FP32 on FP64-formed offsets (as the
 // deformable kernel's mixed path), accumulated per vertex in FP32; torques,
 // ring sums and integration stay FP64.

@@ -528,4 +528,37 @@ __device__ __forceinline__ void reduce_partials(const double* partials, int nblo
   }
 }
 
+// Sums of N arrays over v[f .. f + n) (stride `st` doubles, n <= 256) by one
+// warp, left in v[f], as a tree of neighbours: ((0 + 1) + (2 + 3)) + ..., each
+// lane its own run of 1, 2, 4 or 8 elements first.  The order is that of a tree
+// over shared memory with strides 1, 2, 4, ..: the stiff area term multiplies
+// the rounding of a ring's area by up to 1e5, and in mixed precision positions
+// that differ in their last bits round to other FP32 offsets (with lanes
+// striding over the ring, 200 steps of the 39,424-vertex mixed run ended 1e-9
+// away).
+template <int N>
+__device__ __forceinline__ void ring_sums(double* const (&v)[N], int f, int n, int st = 1) {
+  const int wl = threadIdx.x & 31;
+  const int run = n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : 8;
+  const int c = wl * run;
+  double x[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    const double* e = v[q] + (size_t)f * st;
+    const auto at = [&](int k) { return k < n ? e[k * st] : 0.0; };
+    if (run == 1) x[q] = at(c);
+    else if (run == 2) x[q] = at(c) + at(c + 1);
+    else {
+      x[q] = (at(c) + at(c + 1)) + (at(c + 2) + at(c + 3));
+      if (run == 8) x[q] += (at(c + 4) + at(c + 5)) + (at(c + 6) + at(c + 7));
+    }
+  }
+  for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+    for (int q = 0; q < N; q++) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
+  if (wl == 0)
+#pragma unroll
+    for (int q = 0; q < N; q++) v[q][(size_t)f * st] = x[q];
+}
+
 }  // namespace cr

@@ -59,8 +59,8 @@ template <> struct BoxSel<true> {
   __device__ static const Box& get(const SysParams&, const Box& b) { return b; }
 };
 
-// Every CTA ends in the last-block protocol so that the op counter and the
-// conditional rebuild node of a batch graph see each op exactly once.
+// Every CTA ends in the last-block protocol so that the op counter sees each
+// op exactly once.
 __device__ __forceinline__ void tile_skip(const StepArgs& s, DevStatus* st) {
   if (is_last_block(st)) {
     if (threadIdx.x == 0) {
@@ -612,16 +612,6 @@ __device__ __forceinline__ bool moved_beyond(double2 d, double cut) {
   return 3.0 * dist_of(d) > cut;
 }
 
-// Sum of v[f .. f + n) (stride `st` doubles) by one warp in a fixed order,
-// left in v[f].
-__device__ __forceinline__ void ring_sum(double* v, int f, int n, int st = 1) {
-  const int wl = threadIdx.x & 31;
-  double x = 0.0;
-  for (int q = wl; q < n; q += 32) x += v[(f + q) * st];
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  if (wl == 0) v[f * st] = x;
-}
-
 // The warp's marked slots: in FP64, or (mixed precision) in FP32 unless the
 // slot is near, then in FP64.  The lanes of a warp hold uneven numbers of
 // slots (0.8 on average for the smooth Lennard-Jones run, 3 to 4 for the
@@ -631,7 +621,9 @@ __device__ __forceinline__ void ring_sum(double* v, int f, int n, int st = 1) {
 // evaluates one entry per round, and every lane then adds up the results of
 // its own slots (those with slot % L = its lane) in slot order: the sums do
 // not depend on how the queue was filled or dealt.
-// An entry is own vertex << 24 | slot (staged: | list entry).
+// An entry is own vertex << 24 | slot (staged: | list entry); evaluating it
+// sets kNear where a mixed slot was near.
+constexpr int kNear = 1 << 23;
 template <int QN>
 struct UnitQueue {
   int* q;        // [QN] this warp's entries
@@ -659,6 +651,7 @@ __device__ __forceinline__ void queue_eval(const SysParams& p, const B& bx, cons
       const float len2 = fmaf(sf.y, sf.y, sf.x * sf.x);
       wide = mixed_slot_f32<POT>(p, bx, xi, seg_i, sf, f2(pseg_i), len2, sqrtf(len2), ri, rj, xj, xjq, xjqq, f1, f2_,
                                  en_);
+      if (wide) u.q[e] = w | kNear;
     }
     if (wide)
       smooth_slot_f64<POT>(p, bx, xi, s_pos[lq], seg_i, pseg_i, s_il[lq], ri, rj, xj, xjq, xjqq, f1, f2_, en_);
@@ -668,8 +661,12 @@ __device__ __forceinline__ void queue_eval(const SysParams& p, const B& bx, cons
   }
 }
 
-template <int QN, bool EN>
-__device__ __forceinline__ void queue_add(const UnitQueue<QN>& u, int k, double2& fi, double2& fq, double& ei) {
+// Mixed precision: a vertex's far slots (pass 0) are added before its near
+// ones (pass 1).
+template <int QN, int PREC, bool EN>
+__device__ __forceinline__ void queue_add(const UnitQueue<QN>& u, int k, int pass, double2& fi, double2& fq,
+                                          double& ei) {
+  if (PREC == PREC_MIXED && ((u.q[k] & kNear) != 0) != (pass != 0)) return;
   const double2 f1 = u.fi[k], f2_ = u.fq[k];
   fi.x += f1.x;
   fi.y += f1.y;
@@ -704,7 +701,8 @@ __device__ __forceinline__ void queue_lanes(const SysParams& p, const B& bx, con
     __syncwarp();
     queue_eval<POT, QN, PREC, EN, 32>(p, bx, src, s_pos, s_seg, s_il, s_lp, u, min(QN, total - q0));
     __syncwarp();
-    for (int k = lo; k < hi; k++) queue_add<QN, EN>(u, k - q0, fi, fq, ei);
+    for (int pass = 0; pass < (PREC == PREC_MIXED ? 2 : 1); pass++)
+      for (int k = lo; k < hi; k++) queue_add<QN, PREC, EN>(u, k - q0, pass, fi, fq, ei);
     __syncwarp();
   }
 }
@@ -953,11 +951,10 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     const int nrings = s_tp[nvt - 1].x - s_tp[0].x + 1;
     for (int q = BLOCK / 32 - 1 - t / 32; q < nrings; q += BLOCK / 32) {
       const int f = s_rfirst[q], n = s_tp[f].y >> 16;
-      ring_sum(s_r0, f, n);
+      ring_sums<1>({s_r0}, f, n);
       if constexpr (MODE == MODE_FORCE) {
-        ring_sum(s_r1, f, n);
-        ring_sum(&s_r2[0].x, f, n, 2);
-        ring_sum(&s_r2[0].y, f, n, 2);
+        ring_sums<1>({s_r1}, f, n);
+        ring_sums<2>({&s_r2[0].x, &s_r2[0].y}, f, n, 2);
       }
     }
   }
@@ -1085,8 +1082,16 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
           __syncthreads();
           const int n = s_queued;
           for (int q0 = 0; q0 == 0 || q0 < n; q0 += QC) {
-            if (q0 > 0) {
-              // a queue longer than its space: the next part
+            if (n > QC) {
+              // more entries than the queue holds: in parts, by the entries'
+              // order in the lists (the rounds end in any order), so that every
+              // vertex's slots still come in slot order
+              if (q0 == 0)
+                for (int e = t; e < g->entries; e += BLOCK) {
+                  int at = __popc(s_bal[e / 32] & ((1u << e % 32) - 1u));
+                  for (int w = 0; w < e / 32; w++) at += __popc(s_bal[w]);
+                  g->place[e] = (unsigned short)at;
+                }
               __syncthreads();
               for (int e = t; e < g->entries; e += BLOCK) {
                 const int k = g->place[e] - q0;
@@ -1099,15 +1104,16 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
             __syncthreads();
             // this thread's marked entries, 32 of its run at a time
             const int run = g->start[t], len = g->start[t + 1] - run;
-            for (int b = 0; b < len; b += 32) {
-              const int e0 = run + b;
-              unsigned m = __funnelshift_r(s_bal[e0 / 32], s_bal[e0 / 32 + 1], e0 % 32);
-              if (len - b < 32) m &= (1u << (len - b)) - 1u;
-              for (; m; m &= m - 1u) {
-                const int k = g->place[e0 + __ffs((int)m) - 1] - q0;
-                if (k >= 0 && k < QC) queue_add<QC, kOut>(uq, k, fi64, fq64, ei);
+            for (int pass = 0; pass < (PREC == PREC_MIXED ? 2 : 1); pass++)
+              for (int b = 0; b < len; b += 32) {
+                const int e0 = run + b;
+                unsigned m = __funnelshift_r(s_bal[e0 / 32], s_bal[e0 / 32 + 1], e0 % 32);
+                if (len - b < 32) m &= (1u << (len - b)) - 1u;
+                for (; m; m &= m - 1u) {
+                  const int k = g->place[e0 + __ffs((int)m) - 1] - q0;
+                  if (k >= 0 && k < QC) queue_add<QC, PREC, kOut>(uq, k, pass, fi64, fq64, ei);
+                }
               }
-            }
           }
         }
       }
@@ -1239,7 +1245,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
       if (t < nvt) s_r1[t] = epair;
       __syncthreads();
       for (int q = t / 32; q <= s_tp[nvt - 1].x - s_tp[0].x; q += BLOCK / 32)
-        ring_sum(s_r1, s_rfirst[q], s_tp[s_rfirst[q]].y >> 16);
+        ring_sums<1>({s_r1}, s_rfirst[q], s_tp[s_rfirst[q]].y >> 16);
       __syncthreads();
       if (t < nvt && k == 0) s.p_energy[ring] = s_r1[t];
     }
@@ -1363,7 +1369,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
       if (t < nvt) s_r1[t] = epair;
       __syncthreads();
       for (int q = t / 32; q <= s_tp[nvt - 1].x - s_tp[0].x; q += BLOCK / 32)
-        ring_sum(s_r1, s_rfirst[q], s_tp[s_rfirst[q]].y >> 16);
+        ring_sums<1>({s_r1}, s_rfirst[q], s_tp[s_rfirst[q]].y >> 16);
       __syncthreads();
       if (t < nvt && k == 0) s.p_energy[ring] = s_r1[t];
     }

@@ -308,7 +308,8 @@ int cr_init_vertices_on_particles(cr_ctx* ctx, const double* draws);
 
 /* ---- run statistics and measurement ------------------------------------ */
 /* Kernels this context has run since creation (direct launches and
- * graph-node kernels per replay). */
+ * graph-node kernels per replay; builds that only watch a FIRE sequence and
+ * return at once are not counted). */
 int cr_get_launch_count(const cr_ctx* ctx, long long* out);
 /* The context's CUDA stream (cudaStream_t), for recording timing events. */
 int cr_get_stream(const cr_ctx* ctx, void** out);
@@ -322,15 +323,18 @@ int cr_profile_step_kernel(cr_ctx* ctx, long reps, double* ms_per_launch);
  * tiles hold 128, 96, 64 or 32 vertices of whole rings respectively. */
 int cr_set_lanes(cr_ctx* ctx, int lanes);
 int cr_get_lanes(const cr_ctx* ctx, int* lanes);
-/* 1: step sequences run as captured CUDA graphs (default), every op that
- * moved positions followed by the one-launch rebuild check; 0: direct
- * launches with a host check after each op. */
+/* 1 (default): step sequences go to the stream without host checks between
+ * ops (as a captured CUDA graph where a call replays it at least eight times,
+ * else as plain launches, or in a multi-step kernel), every op that moved
+ * positions followed by the one-launch rebuild check; 0: direct launches with
+ * a host check after each op. */
 int cr_set_use_graphs(cr_ctx* ctx, int on);
 /* 1 (default): the middle steps of NVE, Langevin and BAOAB runs of
- * deformable rings run in a multi-step kernel (up to 64 steps per launch,
- * grid barriers between steps) when the GPU holds all of its CTAs at once
- * and one or two lanes per vertex are in use; 0: one launch per step.  FP64
- * results are identical; mixed-precision results agree to FP32 rounding.
+ * deformable rings, and their FIRE iterations in FP64, run in a multi-step
+ * kernel (up to 64 steps per launch, grid barriers between steps) when the
+ * GPU holds all of its CTAs at once and one or two lanes per vertex are in
+ * use; 0: one launch per op.  FP64
+ * step results are identical, FIRE's agree to rounding; mixed-precision results agree to FP32 rounding.
  * The kernel's grid barriers need all of its CTAs resident (so does the
  * one-launch neighbour-list build).  With other work running on the same
  * GPU a barrier may give up (cr_set_spin_limit); the context then goes back

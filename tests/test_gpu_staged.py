@@ -70,3 +70,30 @@ def test_coordinates_far_out(cuda_device, boxes):
 def test_ring_sizes(cuda_device, nv, lanes):
     pk = synth.make_packing([nv] * 9, [1.0] * 9, 1.05, 0.35 if nv > 10 else 0.06, seed=8, placement="rsa")
     _same(_states(pk, "wca", "vertexSmooth", lanes, dt=2e-4))
+
+
+@pytest.mark.parametrize("interaction", ["vertexVertex", "vertexSmooth"])
+def test_queue_in_parts(cuda_device, interaction):
+    # far out, so that every listed slot is marked: 1,000 entries and more per
+    # tile, several times what the queue holds at once
+    pk = synth.make_packing([30] * 24, [1.0] * 24, 1.05, 0.45, seed=12, placement="rsa")
+    for _ in range(3):  # the marking rounds end in another order each time
+        _same(_states(pk, "harmonic", interaction, 2, cutoff=1.5, shift=9.0e5 * float(pk.box[0])))
+
+
+@pytest.mark.parametrize("nv", [3, 31, 32, 33, 64, 65, 127, 128])
+def test_ring_areas(cuda_device, nv):
+    pk = synth.make_packing([nv] * 3, [1.0] * 3, 1.05, 0.2, seed=13)
+    d = DPM2D.from_packing(pk)
+    d.setLanes(1)
+    d.calcNeighborList(d.setDisplacementCutoff(0.5, 2 * pk.rad.mean()))
+    d.calcForceEnergy()
+    x = pk.pos.reshape(3, nv, 2)
+    x = x - x[:, :1]
+    n = np.roll(x, -1, axis=1)
+    area = 0.5 * np.abs((x[..., 0] * n[..., 1] - x[..., 1] * n[..., 0]).sum(1))
+    # per term and side: two products of up to 4 R^2 and their difference, three
+    # roundings of 2^-53, halved, R^2 = area / pi (2 area 2^-53); the sum adds
+    # as much as 2^-53 area per term: 3 nv 2^-52 area for both sides
+    assert np.abs(d.getAreas() - area).max() <= 4 * nv * 2.0 ** -52 * area.max()
+    d.close()
