@@ -34,7 +34,8 @@ namespace cr {
 // the rotation's sine and cosine once per ring, and no sums over the system
 // are formed (nothing reads them).  100 steps with 4 or 5 rebuilds, one graph
 // captured for them: 98,304 vertices, WCA, FP64, 4.10 -> 2.82 ms; 36,024
-// vertices, FP32 pairs, 2.41 -> 1.97 ms.
+// vertices, FP32 pairs, 2.41 -> 1.97 ms (with calls as plain launches, 2.63 and
+// 1.58 ms).
 template <int POT, int MODE, int BLOCK, int L, int PREC>
 __global__ void __launch_bounds__(BLOCK) k_rigid(const __grid_constant__ SysParams p,
                                                  const __grid_constant__ SysArrays a,
