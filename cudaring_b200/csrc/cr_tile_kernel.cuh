@@ -913,6 +913,9 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     const double2 xn = s_pos[ln];
     const double2 seg = pbc2(bx, xn, x);
     s_seg[t] = seg;
+    // ahead of the barrier: the pair phase reads the predecessor's too, and no
+    // barrier lies between phase 2 and the unstaged pair phase
+    s_il[t] = rsqrt(fma(seg.y, seg.y, seg.x * seg.x));
     const double2 x0 = s_pos[lf];
     const double2 u = pbc2(bx, x, x0);
     const double2 un = pbc2(bx, xn, x0);
@@ -968,7 +971,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
   double esh = 0.0;
   if (t < nvt) {
     // The reference's divisions are taken as products with a few
-    // reciprocals (1/A0, 1/l0 and the segments' 1/l from one rsqrt each),
+    // reciprocals (1/A0, 1/l0 and each segment's 1/l, formed once in phase 1),
     // a rounding-level difference
     const double area = fabs(s_r0[lf]) * 0.5;
     const double inv_a0 = 1.0 / a0r;
@@ -982,9 +985,8 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     fsh.y += 0.5 * gmA * (npd.x);
     esh += (0.5 * p.ea * dA * dA) / nvr;
     const double ps2 = fma(ps.y, ps.y, ps.x * ps.x), ns2 = fma(ns.y, ns.y, ns.x * ns.x);
-    const double r_pl = rsqrt(ps2), r_nl = rsqrt(ns2);  // 1 / |segment|
+    const double r_pl = s_il[lp], r_nl = s_il[t];  // 1 / |segment|
     const double plen = ps2 * r_pl, nlen = ns2 * r_nl;
-    s_il[t] = r_nl;
     const double tl0 = s_l0[t], pl0 = s_l0[lp];
     if (p.monomer == 0) {
       const double inv_tl0 = s_il0[t], inv_pl0 = s_il0[lp];
