@@ -749,6 +749,7 @@ __global__ void __launch_bounds__(BLOCK) k_cg_steps(const __grid_constant__ Diff
     m2 = a.minv[(size_t)3 * v + 2];
   }
   const int l0 = near(-2), l1 = near(-1), l3 = near(1), l4 = near(2);
+  __syncthreads();  // every warp has read its rings' area sums; s_dot is rewritten from here on
   double rr = st0.rr, rz = st0.rz, beta = 0.0, zx = 0.0, zy = 0.0;
   long long iters = st0.iters;
   unsigned long long bar = st0.bar / gridDim.x;
