@@ -117,9 +117,10 @@ struct cr_ctx {
   CgState* cg_state = nullptr;
   double* cg_part = nullptr;   // [148][8] CG reduction partials
   // many iterations per launch (k_cg_steps): pair blocks at list capacity
-  // cgs_cap, tiles, p of the last iteration; cleared when a barrier gave up
+  // cgs_cap, tiles, p of the last iteration, partial sums; cg_steps cleared when
+  // a barrier gave up or there was no memory for them
   double2 *cgs_kxy = nullptr, *cgs_p = nullptr;
-  double* cgs_kyy = nullptr;
+  double *cgs_kyy = nullptr, *cgs_part = nullptr;
   int* cgs_kj = nullptr;
   int2* cgs_tiles = nullptr;
   int cgs_cap = 0, cgs_block = 0, cgs_ntiles = 0;
@@ -1195,7 +1196,7 @@ int cr_destroy(cr_ctx* ctx) {
                   ctx->cell_cnt, ctx->cell_start, ctx->cell_vid, ctx->cell_ring, ctx->cell_pos, ctx->cell_rad,
                   ctx->partials, ctx->status, ctx->fire_state, ctx->p_vel, ctx->p_force, ctx->p_angvel,
                   ctx->diff_f, ctx->diff_e, ctx->diff_dot, ctx->diff_vec, ctx->diff_area, ctx->cg_state,
-                  ctx->cg_part, ctx->cg_minv, ctx->cgs_kxy, ctx->cgs_kyy, ctx->cgs_kj, ctx->cgs_tiles, ctx->cgs_p,
+                  ctx->cg_part, ctx->cg_minv, ctx->cgs_kxy, ctx->cgs_kyy, ctx->cgs_kj, ctx->cgs_tiles, ctx->cgs_p, ctx->cgs_part,
                   ctx->p_torque, ctx->p_moi, ctx->v_torque, ctx->sp_angle, ctx->block_sum, ctx->cell_bucket, ctx->bucket_pos, ctx->bucket_rad,
                   ctx->bucket_ring, ctx->bucket_pq,
                   ctx->prad, ctx->plast, ctx->pid, ctx->pnbr, ctx->pnbr_cnt, ctx->pstatus, ctx->pfire, ctx->pdraws,
@@ -2261,6 +2262,22 @@ extern "C" int cr_param_derivatives(cr_ctx* ctx, int param, double* dU, double* 
   return CR_OK;
 }
 
+// No memory for the scratch of k_cg_steps: one launch per op needs none of it,
+// and holds for the context's later solves too.
+static int cg_steps_drop(cr_ctx* ctx) {
+  cudaGetLastError();
+  ctx->cg_steps = false;
+  for (void* p : {(void*)ctx->cgs_p, (void*)ctx->cgs_part, (void*)ctx->cgs_tiles, (void*)ctx->cgs_kxy,
+                  (void*)ctx->cgs_kyy, (void*)ctx->cgs_kj})
+    if (p) cudaFree(p);
+  ctx->cgs_p = ctx->cgs_kxy = nullptr;
+  ctx->cgs_part = ctx->cgs_kyy = nullptr;
+  ctx->cgs_kj = nullptr;
+  ctx->cgs_tiles = nullptr;
+  ctx->cgs_cap = 0;
+  return CR_OK;
+}
+
 // Scratch and tiles of k_cg_steps; *ok = false where it does not apply (smooth
 // interaction, a grid the GPU does not hold at once, no memory for the rows, a
 // barrier that gave up before).
@@ -2293,21 +2310,18 @@ static int cg_steps_ready(cr_ctx* ctx, bool* ok) {
       if ((int)tiles.size() <= sms) break;
     }
     if (tiles.empty()) return CR_OK;
+    // its own partial sums: the per-op iterations keep theirs (cg_part)
+    if (dalloc(ctx, &ctx->cgs_p, (size_t)2 * ctx->nv) || dalloc(ctx, &ctx->cgs_part, (size_t)8 * tiles.size()) ||
+        dalloc(ctx, &ctx->cgs_tiles, tiles.size()))
+      return cg_steps_drop(ctx);
+    if ((rc = upload(ctx, ctx->cgs_tiles, tiles.data(), tiles.size() * sizeof(int2)))) return rc;
     ctx->cgs_ntiles = (int)tiles.size();
-    if ((rc = dalloc(ctx, &ctx->cgs_p, (size_t)2 * ctx->nv)) ||
-        (rc = dalloc(ctx, &ctx->cg_part, (size_t)8 * std::max(148, ctx->cgs_ntiles))) ||
-        (rc = dalloc(ctx, &ctx->cgs_tiles, tiles.size())) ||
-        (rc = upload(ctx, ctx->cgs_tiles, tiles.data(), tiles.size() * sizeof(int2))))
-      return rc;
   }
   if (cg_steps_max_blocks(ctx->potential, ctx->cgs_block) < ctx->cgs_ntiles) return CR_OK;
   if (ctx->cgs_cap < ctx->cap) {
     const size_t n = (size_t)ctx->cap * ctx->nv;
-    if (dalloc(ctx, &ctx->cgs_kxy, n) || dalloc(ctx, &ctx->cgs_kyy, n) || dalloc(ctx, &ctx->cgs_kj, n)) {
-      cudaGetLastError();  // no room for the rows: one launch per op needs none
-      ctx->cg_steps = false;
-      return CR_OK;
-    }
+    if (dalloc(ctx, &ctx->cgs_kxy, n) || dalloc(ctx, &ctx->cgs_kyy, n) || dalloc(ctx, &ctx->cgs_kj, n))
+      return cg_steps_drop(ctx);
     ctx->cgs_cap = ctx->cap;
   }
   *ok = true;
@@ -2363,12 +2377,13 @@ extern "C" int cr_hessian_solve(cr_ctx* ctx, const double* b, double* x, double 
   if (many) {
     // launches of up to kLaunch iterations each until the state says done
     constexpr int kLaunch = 4096;
-    a.partials = ctx->cg_part;  // cg_steps_ready may have made it larger
+    CgArgs as = a;
+    as.partials = ctx->cgs_part;
     if ((rc = read_status(ctx))) return rc;
     CgSteps ks{ctx->cgs_kxy, ctx->cgs_kyy, ctx->cgs_kj, ctx->cgs_tiles, ctx->cgs_ntiles,
                {ctx->cgs_p, ctx->cgs_p + ctx->nv}, ctx->status_h->spin_limit, kLaunch};
     while (!cs.done && !cs.stalled) {
-      CR_TRY(launch_cg_steps(ctx->stream, ctx->potential, ctx->cgs_block, diff_args(ctx), a, ks));
+      CR_TRY(launch_cg_steps(ctx->stream, ctx->potential, ctx->cgs_block, diff_args(ctx), as, ks));
       ctx->launches++;
       if ((rc = download(ctx, &cs, ctx->cg_state, sizeof(cs)))) return rc;
     }
