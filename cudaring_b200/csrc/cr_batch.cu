@@ -529,7 +529,8 @@ __global__ void k_cclear(DevStatus* st) {
   st->nonfinite = 0;
   st->converged = 0;
   st->done_ctr = 0;
-  st->pbar = 0;
+  st->pbar[0] = st->pbar[1] = 0;
+  st->pturn = 0;
   st->bpending = 0;
 }
 
@@ -812,7 +813,8 @@ int clear_flags(cr_batch* b) {
   b->status_h->nonfinite = 0;
   b->status_h->converged = 0;
   b->status_h->done_ctr = 0;
-  b->status_h->pbar = 0;
+  b->status_h->pbar[0] = b->status_h->pbar[1] = 0;
+  b->status_h->pturn = 0;
   b->status_h->bpending = 0;
   b->status_h->stalled = 0;
   return write_status(b);

@@ -225,13 +225,13 @@ struct DevStatus {
   double sums[8];     // final reductions written by the last block
   unsigned int bar_count;  // grid barrier of the one-launch build: arrivals
   int stalled;        // a grid-barrier wait gave up (the build did not finish)
-  // multi-step kernel (k_tile_steps): barrier counter (arrivals, and above
-  // them the arrivals that asked for a stop), whether a non-finite force was
-  // seen, the counter's upper part before the launch, and the middle steps of
-  // the sequence still to run
-  unsigned long long pbar;
-  int pflag[1];
-  long long pbase;
+  // multi-step kernels: barrier words (cr_bar.h), one in use by a launch while
+  // its CTA 0 clears the other for the next one, and which is next; whether
+  // k_tile_steps saw a non-finite force; the middle steps (or FIRE iterations)
+  // of the sequence still to run
+  unsigned long long pbar[2];
+  int pturn;
+  int pflag;
   long long steps_left;
   // persistent batched FIRE: the last launch left with its force op due
   int bpending;
@@ -251,9 +251,9 @@ __host__ __device__ inline void clear_status_flags(DevStatus& s) {
   s.done_ctr = 0;
   s.bar_count = 0;
   s.stalled = 0;
-  s.pbar = 0;
-  s.pflag[0] = 0;
-  s.pbase = 0;
+  s.pbar[0] = s.pbar[1] = 0;
+  s.pturn = 0;
+  s.pflag = 0;
 }
 
 __device__ __forceinline__ long long barrier_poll_limit(const DevStatus* st) {

@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   if (vs->abort) return;
   const int pending = vs->bpending;  // the last launch left with its force op due
   const int4 tile = a.tiles[blockIdx.x];
+  StepsBarrier bar(st);
   bool stalled = false;
   int rebuild = 0;
   extern __shared__ __align__(16) unsigned char s_stage[];
@@ -44,7 +45,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   for (int j = 0; j < n; j++) {
     if (!(j == 0 && pending)) {
       for (int v = tile.z + threadIdx.x; v < tile.w; v += BLOCK) bfire_prekick(f, v);
-      if (steps_barrier(st) < 0) {
+      if (steps_barrier(bar) < 0) {
         stalled = true;
         break;
       }
@@ -58,7 +59,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
       }
     }
     tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, true, 2>(p, a, s, a.pos, s.pos_out, 0ull, nullptr, j > 0, &g, tile);
-    if (steps_barrier(st) < 0) {
+    if (steps_barrier(bar) < 0) {
       stalled = true;
       break;
     }
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   if (stalled) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->bpending = rebuild;
+    bar.leave();
   }
 }
 

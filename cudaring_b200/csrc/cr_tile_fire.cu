@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   if (left <= 0) return;
   const int n = (int)(left < (long long)s.persist_max ? left : (long long)s.persist_max);
   const bool pending = vs->bpending != 0;  // the last launch left with its force op due
-  const unsigned long long base = (unsigned long long)vs->pbase;
+  StepsBarrier bar(st);
   const long long it0 = vs->fire_iters;
   __shared__ double s_sums[NSUM];
   if (threadIdx.x < NSUM) s_sums[threadIdx.x] = vs->sums[threadIdx.x];
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
         moved |= moved_beyond(pbc2(p, x, s.last_pos[v]), s.disp_cutoff);
       }
       if (moved) st->rebuild = 1;
-      const int b = steps_barrier(st, __syncthreads_or(moved) != 0, base);
+      const int b = steps_barrier(bar, __syncthreads_or(moved) != 0);
       if (b != 0) {
         stalled = b < 0;
         due = b > 0;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
     }
     tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, false, 3>(p, a, s, pos, pos, 0ull, nullptr, j > 0, &g, tile,
                                                                     0.5 * f.dt);
-    if (steps_barrier(st, false, base) < 0) {
+    if (steps_barrier(bar) < 0) {
       stalled = true;
       break;
     }
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   st->ops_done += 2 * done;
   st->steps_left = left - done;
   st->bpending = due ? 1 : 0;
-  st->pbase = (long long)(*(volatile unsigned long long*)&st->pbar >> kBarArrivals);
+  bar.leave();
 }
 
 namespace {

@@ -20,6 +20,7 @@
 #pragma once
 #include <type_traits>
 
+#include "cr_bar.h"
 #include "cr_tile.cuh"
 
 namespace cr {
@@ -1475,18 +1476,13 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
 // non-finite force.
 //
 // Those stop decisions must be the same in every CTA, so they travel with the
-// barrier itself: its 64-bit counter holds the arrivals in the low 40 bits and
-// the arrivals of CTAs that want to stop above them, so the poll that sees the
-// barrier complete brings the decision too (a flag word of its own cost
-// another trip to L2 per step).  The upper count is compared with its value at
-// the start of the launch, which CTA 0 keeps in status.pbase (written after
-// the last barrier of a launch, read by every CTA before the first).  A
-// non-finite force also goes into status.pflag[0].  The step counters
-// (rng_step, ops_done, steps_left, pbase) are read by every CTA before barrier
-// 0 and updated by CTA 0 after the loop.  Every barrier wait is bounded: a CTA
-// that gives up sets stalled and abort and leaves; the others see stalled and
-// leave too.
-constexpr int kBarArrivals = 40;
+// barrier's own word (cr_bar.h): the poll that sees the barrier complete brings
+// the decision too (a flag word of its own cost another trip to L2 per step).
+// The word is one of two that launches take in turn: CTA 0 clears the other one
+// for the next launch.  A non-finite force also goes into status.pflag.  The
+// step counters and the turn are read by every CTA before barrier 0 and updated
+// by CTA 0 after the loop.  Every barrier wait is bounded: a CTA that gives up
+// sets stalled and abort and leaves; the others see stalled and leave too.
 
 __device__ __forceinline__ unsigned long long pst_ld_acquire(const unsigned long long* a) {
   unsigned long long v;
@@ -1500,23 +1496,38 @@ __device__ __forceinline__ unsigned long long pst_atom_add_release(unsigned long
   return old;
 }
 
-// Barrier over the grid on status.pbar (its arrivals a multiple of gridDim.x
-// at launch).  stop: this CTA wants the loop to end (thread 0's value counts).
-// Returns 0: go on, 1: some CTA wanted to stop (the upper count is no longer
-// base), -1: the wait gave up.
-__device__ __forceinline__ int steps_barrier(DevStatus* st, bool stop = false, unsigned long long base = 0ull) {
+// The barriers of one launch.  Every thread of the CTA makes one before the
+// first barrier.
+struct StepsBarrier {
+  DevStatus* st;
+  unsigned long long* word;
+  int turn, k;  // k: barriers passed
+  __device__ __forceinline__ explicit StepsBarrier(DevStatus* s) : st(s), k(0) {
+    turn = *(volatile int*)&s->pturn;
+    word = &s->pbar[turn];
+    if (blockIdx.x == 0 && threadIdx.x == 0) s->pbar[turn ^ 1] = 0ull;
+  }
+  // After the last barrier, by one thread of CTA 0: the next launch takes the
+  // other word.
+  __device__ __forceinline__ void leave() const {
+    if (k > 0) st->pturn = turn ^ 1;
+  }
+};
+
+// Barrier over the grid.  stop: this CTA wants the loop to end (thread 0's
+// value counts).  Returns 0: go on, 1: some CTA wanted to stop, -1: the wait
+// gave up.
+__device__ __forceinline__ int steps_barrier(StepsBarrier& b, bool stop = false) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    constexpr unsigned long long kLow = (1ull << kBarArrivals) - 1ull;
+    DevStatus* st = b.st;
     int ok = 0;
-    const unsigned long long g = gridDim.x;
-    const unsigned long long prev = pst_atom_add_release(&st->pbar, stop ? 1ull | (1ull << kBarArrivals) : 1ull);
-    const unsigned long long target = ((prev & kLow) / g + 1ull) * g;
+    pst_atom_add_release(b.word, bar_arrival(b.k, stop));
     const long long lim = barrier_poll_limit(st);
     long long it = 0;
     unsigned long long now;
-    while (((now = pst_ld_acquire(&st->pbar)) & kLow) < target) {
+    while (!bar_complete(now = pst_ld_acquire(b.word), b.k, gridDim.x)) {
       if (++it > lim || *(volatile int*)&st->stalled) {
         ok = -1;
         break;
@@ -1526,11 +1537,12 @@ __device__ __forceinline__ int steps_barrier(DevStatus* st, bool stop = false, u
     if (ok < 0) {
       atomicExch(&st->stalled, 1);
       atomicExch(&st->abort, 1);
-    } else if ((now >> kBarArrivals) != base) {
+    } else if (bar_stopped(now, b.k)) {
       ok = 1;
     }
     s_ok = ok;
   }
+  b.k++;
   __syncthreads();
   return s_ok;
 }
@@ -1548,7 +1560,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
   if (left <= 0) return;
   const int n = (int)(left < (long long)s.persist_max ? left : (long long)s.persist_max);
   const unsigned long long step0 = (unsigned long long)vs->rng_step;
-  const unsigned long long base = (unsigned long long)vs->pbase;
+  StepsBarrier bar(st);
   double2* pos0 = const_cast<double2*>(a.pos);
   double2* pos1 = s.pos_out;
   extern __shared__ __align__(16) unsigned char s_stage[];
@@ -1561,9 +1573,9 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
     const double2* pin = (j & 1) ? pos1 : pos0;
     double2* pout = (j & 1) ? pos0 : pos1;
     const bool stop = tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC, false, 1>(
-        p, a, s, pin, pout, step0 + (unsigned long long)j, &st->pflag[0], j > 0, &g, tile);
+        p, a, s, pin, pout, step0 + (unsigned long long)j, &st->pflag, j > 0, &g, tile);
     done = j + 1;
-    const int b = steps_barrier(st, stop, base);
+    const int b = steps_barrier(bar, stop);
     if (b < 0) {
       stalled = true;
       break;
@@ -1580,15 +1592,14 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
     for (int v = tile.z + threadIdx.x; v < tile.w; v += BLOCK) pos0[v] = pos1[v];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && done > 0) {
-    if (stopped && *(volatile int*)&st->pflag[0]) {
+    if (stopped && *(volatile int*)&st->pflag) {
       st->nonfinite = 1;
       st->abort = 1;
     }
     st->rng_step += done;
     st->ops_done += done;
     st->steps_left -= done;
-    // the arrivals of the last barrier are all in
-    st->pbase = (long long)(*(volatile unsigned long long*)&st->pbar >> kBarArrivals);
+    bar.leave();
   }
 }
 
