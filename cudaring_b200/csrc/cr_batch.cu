@@ -947,17 +947,19 @@ int add_fire_iterations(cr_batch* b, cudaStream_t st, long n) {
 }
 
 // The persistent FIRE kernel of the batch's configuration, when it has one
-// and the GPU holds all of its CTAs at once; *block its CTA size.
-BFireStepsFn persist_fn(cr_batch* b, int* block) {
-  if (b->no_persist || b->precision != CR_PRECISION_FP64) return nullptr;
-  const int bl = batch_tile_block(b->lanes, b->block);
-  BFireStepsFn fn = bfire_steps_fn(b->potential, inter_kind(b), b->lanes, bl);
-  if (!fn) return nullptr;
-  auto it = b->persist_max.find(fn);
-  if (it == b->persist_max.end()) it = b->persist_max.emplace(fn, bfire_steps_max_blocks(fn, bl)).first;
-  if ((int)b->tiles_h.size() > it->second) return nullptr;
-  *block = bl;
-  return fn;
+// and the GPU holds all of its CTAs at once (else fn is null).
+// With the staged neighbourhood where that grid fits, else without.
+BFireKernel persist_kernel(cr_batch* b) {
+  if (b->no_persist || b->precision != CR_PRECISION_FP64) return {};
+  for (const bool staged : {true, false}) {
+    const BFireKernel k =
+        bfire_kernel(b->potential, inter_kind(b), b->lanes, batch_tile_block(b->lanes, b->block), staged);
+    if (!k.fn) continue;
+    auto it = b->persist_max.find(k.fn);
+    if (it == b->persist_max.end()) it = b->persist_max.emplace(k.fn, bfire_max_blocks(k)).first;
+    if ((int)b->tiles_h.size() <= it->second) return k;
+  }
+  return {};
 }
 
 // FIRE iterations with the persistent kernel onto stream st (capturing or
@@ -965,7 +967,7 @@ BFireStepsFn persist_fn(cr_batch* b, int* block) {
 // (at work when the launch left with a system's displacement check fired),
 // then one launch that only completes a force op left pending, so the chunk
 // ends on a whole iteration.
-int add_fire_persistent(cr_batch* b, cudaStream_t st, int launches, BFireStepsFn fn, int block) {
+int add_fire_persistent(cr_batch* b, cudaStream_t st, int launches, const BFireKernel& k) {
   StepArgs s = step_args(b);
   s.kind = KIND_FIRE;
   s.advance = 0;
@@ -974,11 +976,11 @@ int add_fire_persistent(cr_batch* b, cudaStream_t st, int launches, BFireStepsFn
   s.use_cond = 0;
   const SysParams p = with_f32_constants(b->p);
   for (int i = 0; i < launches; i++) {
-    launch_bfire_steps(fn, tile_cfg(b, st), block, p, arrays(b), s, bfire_args(b), 64);
+    launch_bfire_steps(k, tile_cfg(b, st), p, arrays(b), s, bfire_args(b), 64);
     b->launches++;
     enqueue_build(b, st, 0);
   }
-  launch_bfire_steps(fn, tile_cfg(b, st), block, p, arrays(b), s, bfire_args(b), 0);
+  launch_bfire_steps(k, tile_cfg(b, st), p, arrays(b), s, bfire_args(b), 0);
   b->launches++;
   BT_TRY(cudaGetLastError());
   return CR_OK;
@@ -1028,8 +1030,7 @@ int fire_loop(cr_batch* b, long maxIter, long* done_out) {
   // persistent FIRE: chunks of up to 16 x 64 iterations; every system stops at
   // its iteration limit (fire_cap, set by the caller), so the loop ends when
   // every system has converged or reached it
-  int block = 0;
-  while (BFireStepsFn fn = persist_fn(b, &block)) {
+  for (BFireKernel k = persist_kernel(b); k.fn; k = persist_kernel(b)) {
     if ((rc = pull_sys(b))) return rc;
     bool any = false;
     for (const BatchSys& s : b->bsys_h) any = any || (s.active && !s.converged);
@@ -1043,7 +1044,7 @@ int fire_loop(cr_batch* b, long maxIter, long* done_out) {
     for (const BatchSys& s : b->bsys_h)
       if (s.active && !s.converged) left = std::max(left, s.fire_cap - s.fire_iters);
     const int launches = (int)std::min<long long>(16, (left + 63) / 64 + 1);
-    if ((rc = add_fire_persistent(b, b->stream, launches, fn, block))) return rc;
+    if ((rc = add_fire_persistent(b, b->stream, launches, k))) return rc;
     if ((rc = read_status(b))) return rc;
     if (b->status_h->abort) {
       if (b->status_h->nonfinite) return b->fail(CR_ENONFINITE, "non-finite force in a batched FIRE run");
@@ -1184,8 +1185,8 @@ int compress_body(cr_batch* b, CompArgs a, cudaGraph_t outer_body) {
   cudaGraph_t inner_body;
   if ((rc = add_while(b, s2, a.inner, &inner_body))) return rc;
   BT_TRY(cudaStreamBeginCaptureToGraph(s3, inner_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  int block = 0;
-  if (BFireStepsFn fn = persist_fn(b, &block)) rc = add_fire_persistent(b, s3, 4, fn, block);
+  const BFireKernel k = persist_kernel(b);
+  if (k.fn) rc = add_fire_persistent(b, s3, 4, k);
   else rc = add_fire_iterations(b, s3, 64);
   if (!rc) k_cfire_more<<<1, 256, 0, s3>>>(a);
   cudaGraph_t ib_out;

@@ -97,9 +97,14 @@ __device__ __forceinline__ void bfire_prekick(const BFire& f, int v) {
 // configuration has none (FP64 only; tile shapes (1, 128) and (2, 192)).
 // nmax = 0 only completes a force op left pending by the last launch.
 using BFireStepsFn = void (*)(SysParams, SysArrays, StepArgs, BFire, int);
-BFireStepsFn bfire_steps_fn(int pot, int inter, int lanes, int block);
-int bfire_steps_max_blocks(BFireStepsFn fn, int block);
-void launch_bfire_steps(BFireStepsFn fn, const LaunchCfg& c, int block, const SysParams& p, const SysArrays& a,
+struct BFireKernel {
+  BFireStepsFn fn = nullptr;
+  int block = 0;     // threads per CTA
+  size_t smem = 0;   // dynamic shared memory (the stage; 0: the form without one)
+};
+BFireKernel bfire_kernel(int pot, int inter, int lanes, int block, bool staged);
+int bfire_max_blocks(const BFireKernel& k);   // CTAs the device holds at once
+void launch_bfire_steps(const BFireKernel& k, const LaunchCfg& c, const SysParams& p, const SysArrays& a,
                         const StepArgs& s, const BFire& f, int nmax);
 
 }  // namespace cr

@@ -717,14 +717,23 @@ int launch_chunk(cr_ctx* ctx, const std::vector<Op>& ops, int kind, long n, size
 constexpr int kStepsPerLaunch = 64;
 constexpr int kStepsLaunches = 16;
 
-bool steps_eligible(cr_ctx* ctx, int kind) {
-  if (!ctx->multistep || !ctx->use_graphs) return false;
-
-  if (ctx->shape == CR_SHAPE_RIGID) return false;
-  if (kind != KIND_NVE && kind != KIND_LANGEVIN && kind != KIND_BAOAB) return false;
-  if (ctx->lanes != 1 && ctx->lanes != 2) return false;
-  const int maxb = tile_steps_max_blocks(ctx->potential, inter_kind(ctx), ctx->lanes, ctx->precision);
-  return maxb >= (int)ctx->tiles_h.size();
+// Which form of k_tile_steps serves the run: with the staged neighbourhood where
+// the GPU holds its grid at once, else without it where it holds that one (one
+// lane per vertex; rings of 97 to 128 vertices have no other choice).  One lane,
+// tiles of 100 vertices, us per step with a rebuild in 40 to 50, unstaged form
+// against one launch per op: smooth 445 tiles 8.7 / 13.5, 592 tiles 9.9 / 14.4;
+// vertex-vertex 593 tiles 8.2 / 12.4, 740 tiles 9.9 / 13.2.
+enum class Steps { none, staged, unstaged };
+Steps steps_form(cr_ctx* ctx, int kind) {
+  if (!ctx->multistep || !ctx->use_graphs) return Steps::none;
+  if (ctx->shape == CR_SHAPE_RIGID) return Steps::none;
+  if (kind != KIND_NVE && kind != KIND_LANGEVIN && kind != KIND_BAOAB) return Steps::none;
+  if (ctx->lanes != 1 && ctx->lanes != 2) return Steps::none;
+  const int tiles = (int)ctx->tiles_h.size();
+  for (const bool staged : {true, false})
+    if (tile_steps_max_blocks(ctx->potential, inter_kind(ctx), ctx->lanes, ctx->precision, staged) >= tiles)
+      return staged ? Steps::staged : Steps::unstaged;
+  return Steps::none;
 }
 
 // `launches` multi-step launches, each with the build that may follow it.
@@ -732,7 +741,7 @@ bool steps_eligible(cr_ctx* ctx, int kind) {
 // microseconds, so the host is ahead of it anyway, while a graph of them had
 // to be captured, instantiated and destroyed again for every sequence whose
 // parameters had changed (0.3 to 0.5 ms of a 200-step call).
-int launch_steps(cr_ctx* ctx, int kind, int b, int launches) {
+int launch_steps(cr_ctx* ctx, int kind, Steps form, int b, int launches) {
   StepArgs s = base_args(ctx);
   s.kind = kind;
   s.pos_out = ctx->pos[b ^ 1];
@@ -748,7 +757,7 @@ int launch_steps(cr_ctx* ctx, int kind, int b, int launches) {
   nb.count_update = 1;
   const int fb = nbr_fused_blocks(ctx->nv, ctx->fused_max);
   for (int r = 0; r < launches; r++) {
-    CR_TRY(launch_tile_steps(c, ctx->potential, inter_kind(ctx), ctx->p, a, s));
+    CR_TRY(launch_tile_steps(c, ctx->potential, inter_kind(ctx), form == Steps::staged, ctx->p, a, s));
     launch_nbr_fused(ctx->stream, ctx->p, ctx->grid, nb, fb, 0, true);
     ctx->launches += 2;
   }
@@ -818,7 +827,7 @@ int rerun_degraded(cr_ctx* ctx, int b0, int kind, long nsteps) {
   return run_ops(ctx, kind, nsteps);
 }
 
-int run_steps(cr_ctx* ctx, int kind, long nsteps) {
+int run_steps(cr_ctx* ctx, int kind, Steps form, long nsteps) {
   int rc;
   int b = ctx->cur;
   const int b0 = b;
@@ -839,7 +848,7 @@ int run_steps(cr_ctx* ctx, int kind, long nsteps) {
         left <= 0 ? 0
                   : (int)std::min<long long>(kStepsLaunches,
                                              std::max<long long>(2, (left + kStepsPerLaunch - 1) / kStepsPerLaunch + 1));
-    if (launches && (rc = launch_steps(ctx, kind, b, launches))) return rc;
+    if (launches && (rc = launch_steps(ctx, kind, form, b, launches))) return rc;
     // final op: forces at the last positions and the second half kick; it
     // does nothing while middle steps are left
     enqueue_op(ctx, ctx->stream, Op{OP_TILE, b, b, 0, 0, b}, kind, false, 0, true);
@@ -879,7 +888,7 @@ FireStepsFn fire_steps_eligible(cr_ctx* ctx, int kind) {
   if (kind != KIND_FIRE || !ctx->multistep || !ctx->use_graphs || ctx->shape == CR_SHAPE_RIGID) return nullptr;
   if (ctx->precision != CR_PRECISION_FP64 || ctx->particle == CR_PARTICLE_ACTIVE) return nullptr;
   FireStepsFn fn = fire_steps_fn(ctx->potential, inter_kind(ctx), ctx->lanes);
-  return fire_steps_max_blocks(fn, ctx->lanes) >= (int)ctx->tiles_h.size() ? fn : nullptr;
+  return fire_steps_max_blocks(fn, inter_kind(ctx), ctx->lanes) >= (int)ctx->tiles_h.size() ? fn : nullptr;
 }
 
 int run_fire_steps(cr_ctx* ctx, FireStepsFn fn, long nsteps) {
@@ -902,7 +911,7 @@ int run_fire_steps(cr_ctx* ctx, FireStepsFn fn, long nsteps) {
     const int launches =
         (int)std::min<long long>(kStepsLaunches, std::max<long long>(2, (left + kStepsPerLaunch - 1) / kStepsPerLaunch + 1));
     for (int r = 0; r < launches; r++) {
-      CR_TRY(launch_fire_steps(fn, c, ctx->p, arrays(ctx, b), s, ctx->fp, ctx->fire_state));
+      CR_TRY(launch_fire_steps(fn, inter_kind(ctx), c, ctx->p, arrays(ctx, b), s, ctx->fp, ctx->fire_state));
       launch_nbr_fused(ctx->stream, ctx->p, ctx->grid, nb, nbr_fused_blocks(ctx->nv, ctx->fused_max), 0, true);
       ctx->launches += 2;
     }
@@ -954,7 +963,8 @@ int run_ops(cr_ctx* ctx, int kind, long nsteps) {
     ctx->launches++;
     CR_TRY(cudaGetLastError());
   }
-  if (steps_eligible(ctx, kind)) return run_steps(ctx, kind, nsteps);
+  const Steps form = steps_form(ctx, kind);
+  if (form != Steps::none) return run_steps(ctx, kind, form, nsteps);
   if (FireStepsFn fn = fire_steps_eligible(ctx, kind)) return run_fire_steps(ctx, fn, nsteps);
   if ((rc = clear_flags(ctx))) return rc;
   const long chunk = 128;

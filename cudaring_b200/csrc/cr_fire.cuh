@@ -54,8 +54,8 @@ __device__ __forceinline__ void fire_move(const FireScalars& f, bool rollback, d
 // than one and two.
 using FireStepsFn = void (*)(SysParams, SysArrays, StepArgs, FireParams, double*);
 FireStepsFn fire_steps_fn(int pot, int inter, int lanes);
-int fire_steps_max_blocks(FireStepsFn fn, int lanes);
-cudaError_t launch_fire_steps(FireStepsFn fn, const LaunchCfg& c, const SysParams& p, const SysArrays& a,
+int fire_steps_max_blocks(FireStepsFn fn, int inter, int lanes);
+cudaError_t launch_fire_steps(FireStepsFn fn, int inter, const LaunchCfg& c, const SysParams& p, const SysArrays& a,
                               const StepArgs& s, const FireParams& fp, double* fire_state);
 
 }  // namespace cr

@@ -47,50 +47,54 @@ int tile_vertices(int lanes) { return lanes >= 4 ? 256 / lanes : (lanes == 2 ? 9
 
 
 // Multi-step kernel (k_tile_steps) for one or two lanes per vertex; nullptr
-// for other lane counts.
+// for other lane counts.  Without the stage only for one lane: with two,
+// registers hold three CTAs an SM either way.
 template <int POT, int INTER>
-static TileStepsFn steps_fn_l(int lanes) {
-  if (lanes == 1) return k_tile_steps<POT, INTER, 128, 1, PREC_FP64>;
-  if (lanes == 2) return k_tile_steps<POT, INTER, 192, 2, PREC_FP64>;
+static TileStepsFn steps_fn_l(int lanes, bool staged) {
+  if (lanes == 1) {
+    if (staged) return k_tile_steps<POT, INTER, 128, 1, PREC_FP64, true>;
+    return k_tile_steps<POT, INTER, 128, 1, PREC_FP64, false>;
+  }
+  if (lanes == 2 && staged) return k_tile_steps<POT, INTER, 192, 2, PREC_FP64, true>;
   return nullptr;
 }
 
-TileStepsFn tile_steps_fn_fp64(int pot, int inter, int lanes) {
-  const bool vv = inter == INT_VV;
+template <int POT>
+static TileStepsFn steps_fn_p(int inter, int lanes, bool staged) {
+  return inter == INT_VV ? steps_fn_l<POT, INT_VV>(lanes, staged) : steps_fn_l<POT, INT_SMOOTH>(lanes, staged);
+}
+
+TileStepsFn tile_steps_fn_fp64(int pot, int inter, int lanes, bool staged) {
   switch (pot) {
-    case POT_HARMONIC: return vv ? steps_fn_l<POT_HARMONIC, INT_VV>(lanes) : steps_fn_l<POT_HARMONIC, INT_SMOOTH>(lanes);
-    case POT_LJ: return vv ? steps_fn_l<POT_LJ, INT_VV>(lanes) : steps_fn_l<POT_LJ, INT_SMOOTH>(lanes);
-    case POT_ADHESIVE: return vv ? steps_fn_l<POT_ADHESIVE, INT_VV>(lanes) : steps_fn_l<POT_ADHESIVE, INT_SMOOTH>(lanes);
-    case POT_WCA: return vv ? steps_fn_l<POT_WCA, INT_VV>(lanes) : steps_fn_l<POT_WCA, INT_SMOOTH>(lanes);
+    case POT_HARMONIC: return steps_fn_p<POT_HARMONIC>(inter, lanes, staged);
+    case POT_LJ: return steps_fn_p<POT_LJ>(inter, lanes, staged);
+    case POT_ADHESIVE: return steps_fn_p<POT_ADHESIVE>(inter, lanes, staged);
+    case POT_WCA: return steps_fn_p<POT_WCA>(inter, lanes, staged);
     default: return nullptr;
   }
 }
 
-static TileStepsFn steps_fn(int pot, int inter, int lanes, int precision) {
-  return precision == CR_PRECISION_MIXED ? tile_steps_fn_mixed(pot, inter, lanes) : tile_steps_fn_fp64(pot, inter, lanes);
+static TileStepsFn steps_fn(int pot, int inter, int lanes, int precision, bool staged) {
+  return precision == CR_PRECISION_MIXED ? tile_steps_fn_mixed(pot, inter, lanes, staged)
+                                         : tile_steps_fn_fp64(pot, inter, lanes, staged);
 }
 
-// the staged neighbourhood (cr_tile_kernel.cuh)
-static size_t steps_smem(int lanes) { return lanes == 1 ? stage_bytes<128>() : stage_bytes<96>(); }
-
-int tile_steps_max_blocks(int pot, int inter, int lanes, int precision) {
-  TileStepsFn k = steps_fn(pot, inter, lanes, precision);
-  if (!k) return 0;
-  int dev = 0, sms = 0, occ = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  const size_t smem = steps_smem(lanes);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, lanes == 1 ? 128 : 192, smem) != cudaSuccess) return 0;
-  return occ * sms;
+static size_t steps_smem(int inter, int lanes, bool staged) {
+  return staged ? stage_smem(inter, lanes == 1 ? 128 : 96) : 0;
 }
 
-cudaError_t launch_tile_steps(const LaunchCfg& c, int pot, int inter, const SysParams& p_in, const SysArrays& a,
-                              const StepArgs& s) {
-  TileStepsFn k = steps_fn(pot, inter, c.lanes, c.precision);
+int tile_steps_max_blocks(int pot, int inter, int lanes, int precision, bool staged) {
+  return resident_ctas(steps_fn(pot, inter, lanes, precision, staged), lanes == 1 ? 128 : 192,
+                       steps_smem(inter, lanes, staged));
+}
+
+cudaError_t launch_tile_steps(const LaunchCfg& c, int pot, int inter, bool staged, const SysParams& p_in,
+                              const SysArrays& a, const StepArgs& s) {
+  TileStepsFn k = steps_fn(pot, inter, c.lanes, c.precision, staged);
   if (!k) return cudaErrorInvalidValue;
   const SysParams p = with_f32_constants(p_in);
-  return launch_k(c.pdl, k, dim3(c.grid), dim3(c.lanes == 1 ? 128 : 192), c.stream, steps_smem(c.lanes), p, a, s);
+  return launch_k(c.pdl, k, dim3(c.grid), dim3(c.lanes == 1 ? 128 : 192), c.stream,
+                  steps_smem(inter, c.lanes, staged), p, a, s);
 }
 
 }  // namespace cr

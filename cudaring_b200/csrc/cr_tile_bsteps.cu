@@ -22,7 +22,7 @@
 
 namespace cr {
 
-template <int POT, int INTER, int BLOCK, int L>
+template <int POT, int INTER, int BLOCK, int L, bool STAGED>
 __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / BLOCK)
     k_bfire_steps(const __grid_constant__ SysParams p, const __grid_constant__ SysArrays a,
                   const __grid_constant__ StepArgs s, const __grid_constant__ BFire f, int nmax) {
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
   extern __shared__ __align__(16) unsigned char s_stage[];
   Stage<BLOCK / L> g(s_stage);
   const int n = nmax > 0 ? nmax : pending;
-  if (n > 0) {
+  if (STAGED && n > 0) {
     const BatchSys& bs = s.bsys[tile.x];
     stage_build<INTER, BLOCK, L>(p, bs.box, a, tile, s.last_pos, bs.disp_cutoff, pot_range_f<POT>(p), g);
   }
@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
         break;
       }
     }
-    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, true, 2>(p, a, s, a.pos, s.pos_out, 0ull, nullptr, j > 0, &g, tile);
+    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, true, 2, STAGED>(p, a, s, a.pos, s.pos_out, 0ull, nullptr, j > 0, &g,
+                                                                           tile);
     if (steps_barrier(bar) < 0) {
       stalled = true;
       break;
@@ -78,44 +79,44 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
 
 namespace {
 
-// dynamic shared memory of the two shapes (tiles of 128 and 96 vertices)
-size_t stage_smem(int block) { return block == 128 ? stage_bytes<128>() : stage_bytes<96>(); }
-
-template <int POT, int INTER>
+// Without the stage only for smooth pairs, whose staged form leaves two CTAs an
+// SM (296 tiles); the vertex-vertex kernels hold as many with it (592 with one
+// lane, 444 with two).  us per iteration (calls of 200, list build included),
+// unstaged against one launch per op: one lane, 592 tiles 26.7 / 35.0; two
+// lanes, 444 tiles 25.7 / 33.5; staged, 296 tiles: 23.0 / 32.6 and 22.5 / 32.7.
+template <int POT, int INTER, bool STAGED>
 BFireStepsFn fn_shape(int lanes, int block) {
-  if (lanes == 1 && block == 128) return k_bfire_steps<POT, INTER, 128, 1>;
-  if (lanes == 2 && block == 192) return k_bfire_steps<POT, INTER, 192, 2>;
+  if (lanes == 1 && block == 128) return k_bfire_steps<POT, INTER, 128, 1, STAGED>;
+  if (lanes == 2 && block == 192) return k_bfire_steps<POT, INTER, 192, 2, STAGED>;
   return nullptr;
 }
 
-template <int INTER>
-BFireStepsFn fn_inter(int pot, int lanes, int block) {
-  switch (pot) {
-    case POT_HARMONIC: return fn_shape<POT_HARMONIC, INTER>(lanes, block);
-    case POT_LJ: return fn_shape<POT_LJ, INTER>(lanes, block);
-    case POT_ADHESIVE: return fn_shape<POT_ADHESIVE, INTER>(lanes, block);
-    default: return fn_shape<POT_WCA, INTER>(lanes, block);
-  }
+template <int POT>
+BFireStepsFn fn_pot(int inter, int lanes, int block, bool staged) {
+  if (inter == INT_VV) return staged ? fn_shape<POT, INT_VV, true>(lanes, block) : nullptr;
+  return staged ? fn_shape<POT, INT_SMOOTH, true>(lanes, block) : fn_shape<POT, INT_SMOOTH, false>(lanes, block);
 }
 
 }  // namespace
 
-BFireStepsFn bfire_steps_fn(int pot, int inter, int lanes, int block) {
-  return inter == INT_VV ? fn_inter<INT_VV>(pot, lanes, block) : fn_inter<INT_SMOOTH>(pot, lanes, block);
+BFireKernel bfire_kernel(int pot, int inter, int lanes, int block, bool staged) {
+  BFireKernel k;
+  switch (pot) {
+    case POT_HARMONIC: k.fn = fn_pot<POT_HARMONIC>(inter, lanes, block, staged); break;
+    case POT_LJ: k.fn = fn_pot<POT_LJ>(inter, lanes, block, staged); break;
+    case POT_ADHESIVE: k.fn = fn_pot<POT_ADHESIVE>(inter, lanes, block, staged); break;
+    default: k.fn = fn_pot<POT_WCA>(inter, lanes, block, staged); break;
+  }
+  k.block = block;
+  k.smem = staged ? stage_smem(inter, block == 128 ? 128 : 96) : 0;
+  return k;
 }
 
-int bfire_steps_max_blocks(BFireStepsFn fn, int block) {
-  int dev = 0, sms = 0, occ = 0;
-  if (!fn || cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem(block)) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, stage_smem(block)) != cudaSuccess) return 0;
-  return occ * sms;
-}
+int bfire_max_blocks(const BFireKernel& k) { return resident_ctas(k.fn, k.block, k.smem); }
 
-void launch_bfire_steps(BFireStepsFn fn, const LaunchCfg& c, int block, const SysParams& p, const SysArrays& a,
+void launch_bfire_steps(const BFireKernel& k, const LaunchCfg& c, const SysParams& p, const SysArrays& a,
                         const StepArgs& s, const BFire& f, int nmax) {
-  fn<<<c.grid, block, stage_smem(block), c.stream>>>(p, a, s, f, nmax);
+  k.fn<<<c.grid, k.block, k.smem, c.stream>>>(p, a, s, f, nmax);
 }
 
 }  // namespace cr

@@ -69,8 +69,8 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
         break;
       }
     }
-    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, false, 3>(p, a, s, pos, pos, 0ull, nullptr, j > 0, &g, tile,
-                                                                    0.5 * f.dt);
+    tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC_FP64, false, 3, true>(p, a, s, pos, pos, 0ull, nullptr, j > 0, &g,
+                                                                          tile, 0.5 * f.dt);
     if (steps_barrier(bar) < 0) {
       stalled = true;
       break;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC_FP64, L>() / B
 
 namespace {
 
-size_t fire_smem(int lanes) { return lanes == 1 ? stage_bytes<128>() : stage_bytes<96>(); }
+size_t fire_smem(int inter, int lanes) { return stage_smem(inter, lanes == 1 ? 128 : 96); }
 
 template <int POT, int INTER>
 FireStepsFn fn_lanes(int lanes) {
@@ -129,20 +129,14 @@ FireStepsFn fire_steps_fn(int pot, int inter, int lanes) {
   return inter == INT_VV ? fn_pot<INT_VV>(pot, lanes) : fn_pot<INT_SMOOTH>(pot, lanes);
 }
 
-int fire_steps_max_blocks(FireStepsFn fn, int lanes) {
-  int dev = 0, sms = 0, occ = 0;
-  if (!fn || cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  const size_t smem = fire_smem(lanes);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, lanes == 1 ? 128 : 192, smem) != cudaSuccess) return 0;
-  return occ * sms;
+int fire_steps_max_blocks(FireStepsFn fn, int inter, int lanes) {
+  return resident_ctas(fn, lanes == 1 ? 128 : 192, fire_smem(inter, lanes));
 }
 
-cudaError_t launch_fire_steps(FireStepsFn fn, const LaunchCfg& c, const SysParams& p_in, const SysArrays& a,
+cudaError_t launch_fire_steps(FireStepsFn fn, int inter, const LaunchCfg& c, const SysParams& p_in, const SysArrays& a,
                               const StepArgs& s, const FireParams& fp, double* fire_state) {
   const SysParams p = with_f32_constants(p_in);
-  return launch_k(c.pdl, fn, dim3(c.grid), dim3(c.lanes == 1 ? 128 : 192), c.stream, fire_smem(c.lanes), p, a, s, fp,
+  return launch_k(c.pdl, fn, dim3(c.grid), dim3(c.lanes == 1 ? 128 : 192), c.stream, fire_smem(inter, c.lanes), p, a, s, fp,
                   fire_state);
 }
 

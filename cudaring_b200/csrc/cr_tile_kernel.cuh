@@ -199,7 +199,10 @@ __device__ __forceinline__ bool slot_may_contribute(const MarkBox& m, uint2 ui, 
 // the touched positions into shared memory once and the pair phase reads
 // shared memory alone.  The values read are the same, so no result changes.
 // A tile that touches more rings, vertices or list entries than the stage
-// holds reads global memory as before.
+// holds reads global memory as before, and so does every tile of a grid that
+// the GPU holds at once only without the stage's 31 to 34 KB a CTA (STAGED
+// false: one lane per vertex, 445 to 592 tiles with smooth pairs, 593 to 740
+// with vertex-vertex pairs).
 //   Measured, with the queue of marked slots and the fixed-point marking below
 // (39,424 vertices, smooth Lennard-Jones, FP64, us per step): 17.3 -> 12.1
 // without rebuilds, 18.6 -> 13.9 with one in 20 steps; 9,495 vertices, smooth
@@ -208,10 +211,28 @@ __device__ __forceinline__ bool slot_may_contribute(const MarkBox& m, uint2 ui, 
 constexpr int kStageRings = 128;    // hash slots
 constexpr int kStageHalo = 512;     // touched vertices of other tiles (own and touched: below 1024)
 constexpr int kStageEntries = 1536; // list entries of the tile
-template <int TV>
+template <int TV, int INTER>
 constexpr size_t stage_bytes() {
   return (size_t)(TV + kStageHalo) * (sizeof(double2) + sizeof(double) + sizeof(uint2)) +
-         (size_t)(kStageEntries + kStageHalo + 2 * TV + 4) * sizeof(int) + kStageEntries * 3;
+         (size_t)(kStageEntries + kStageHalo + 2 * TV + 4) * sizeof(int) +
+         kStageEntries * (INTER == INT_SMOOTH ? 3 : 1);  // vertex-vertex pairs have no queue
+}
+
+inline size_t stage_smem(int inter, int tile_vertices) {
+  if (inter == INT_VV) return tile_vertices == 128 ? stage_bytes<128, INT_VV>() : stage_bytes<96, INT_VV>();
+  return tile_vertices == 128 ? stage_bytes<128, INT_SMOOTH>() : stage_bytes<96, INT_SMOOTH>();
+}
+
+// CTAs of a kernel with grid barriers that the current device holds at once (0
+// without one); also allows the kernel that much dynamic shared memory.
+template <typename Fn>
+inline int resident_ctas(Fn* fn, int block, size_t smem) {
+  int dev = 0, sms = 0, occ = 0;
+  if (!fn || cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, smem) != cudaSuccess) return 0;
+  return occ * sms;
 }
 
 // The list entries are in the order of the threads that collect them (own
@@ -225,8 +246,8 @@ struct Stage {
   unsigned* list;  // [kStageEntries] local indices of a neighbour and its two predecessors, 10 bits each
   int* vtx;      // [kStageHalo] global vertex of each touched one
   int* start;    // [TV L + 1] first list entry of each thread
-  unsigned short* place; // [kStageEntries] place of each marked entry in the queue
   unsigned char* owner;  // [kStageEntries] thread of each list entry
+  unsigned short* place; // [kStageEntries] smooth: place of each marked entry in the queue
   int n;         // touched vertices
   int entries;   // list entries
   bool on;       // the tile's neighbourhood fits
@@ -237,8 +258,8 @@ struct Stage {
     list = reinterpret_cast<unsigned*>(u + TV + kStageHalo);
     vtx = reinterpret_cast<int*>(list + kStageEntries);
     start = vtx + kStageHalo;
-    place = reinterpret_cast<unsigned short*>(start + 2 * TV + 4);
-    owner = reinterpret_cast<unsigned char*>(place + kStageEntries);
+    owner = reinterpret_cast<unsigned char*>(start + 2 * TV + 4);
+    place = reinterpret_cast<unsigned short*>(owner + kStageEntries);
     n = entries = 0;
     on = false;
   }
@@ -790,8 +811,9 @@ __device__ __forceinline__ void join_first(int sync) {
 // and the last-block protocol left to the caller; 2 the persistent batched
 // FIRE kernel: plain position loads, everything else as for one op; 3 the FIRE
 // kernel of one system: the CTA's partial sums are all it leaves (fire_hdt:
-// half the time step).  reuse: not the kernel's first op.
-template <int POT, int INTER, int MODE, int BLOCK, int L, int PREC, bool BATCH, int PERSIST>
+// half the time step).  reuse: not the kernel's first op.  STAGED: the
+// persistent kernel has a stage (g).
+template <int POT, int INTER, int MODE, int BLOCK, int L, int PREC, bool BATCH, int PERSIST, bool STAGED>
 __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a, const StepArgs& s,
                                           const double2* __restrict__ pin, double2* __restrict__ pout,
                                           unsigned long long step, int* pflag, bool reuse,
@@ -801,15 +823,17 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
   // write_out = accumulate = 0), so its energy terms are left out at compile time
   constexpr bool kOut = PERSIST != 1;
   constexpr int TS = (MODE == MODE_STEP) ? TV : 1;
-  constexpr bool kStagedSmooth = PERSIST != 0 && INTER == INT_SMOOTH;
-  __shared__ double2 s_own[PERSIST != 0 ? 1 : TV];
-  double2* const s_pos = PERSIST != 0 ? g->x : s_own;
+  static_assert(!STAGED || PERSIST != 0, "one op per launch has no stage");
+  constexpr bool kStagedSmooth = STAGED && INTER == INT_SMOOTH;
+  __shared__ double2 s_own[STAGED ? 1 : TV];
+  double2* s_pos = s_own;
+  if constexpr (STAGED) s_pos = g->x;
   __shared__ double2 s_seg[TV];     // pbc(pos[next] - pos[v])
   __shared__ double s_theta[TV];
   __shared__ double s_l0[TV];       // rest length of segment v -> next(v)
   __shared__ double s_il0[TV];      // its reciprocal
   __shared__ double s_th0[TV];      // rest angle at v
-  __shared__ double s_il[TV];       // 1 / length of segment v -> next(v)
+  __shared__ double s_il[INTER == INT_SMOOTH ? TV : 1];  // 1 / length of segment v -> next(v)
   __shared__ double s_r0[TV];       // shoelace terms -> ring area
   __shared__ double s_r1[TV];       // segment lengths -> perimeter
   __shared__ double2 s_r2[TV];      // offsets from the first vertex -> centroid
@@ -821,10 +845,10 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
   __shared__ int s_lp[TV];
   __shared__ int2 s_tp[TV];         // topology word (ring, k | nv << 16)
   __shared__ int s_rfirst[TV];      // first vertex of each ring of the tile
-  // queue of FP64 smooth units, one part per warp (see queue_units)
+  // queue of FP64 smooth units, one part per warp (see queue_eval)
   constexpr int QN = INTER != INT_SMOOTH ? 1 : (TV > 128 ? 32 : 64);  // 32: the 48 KB of static shared memory
   __shared__ int s_q[BLOCK / 32][QN];
-  __shared__ OwnUnit s_ou[PERSIST != 0 && INTER == INT_SMOOTH ? TV : 1];
+  __shared__ OwnUnit s_ou[kStagedSmooth ? TV : 1];
   __shared__ double2 s_qi[BLOCK / 32][QN], s_qq[BLOCK / 32][QN];
   __shared__ double s_qe[kOut ? BLOCK / 32 : 1][QN];
   __shared__ double s_a0[TV];       // rest area of the vertex's ring
@@ -835,7 +859,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
   __shared__ bool s_syslast;
   __shared__ int s_far;             // a staged coordinate beyond box_frac's range
   __shared__ int s_round;           // marking rounds handed out
-  constexpr int NR = PERSIST != 0 && INTER == INT_SMOOTH ? kStageEntries / 32 : 1;
+  constexpr int NR = kStagedSmooth ? kStageEntries / 32 : 1;
   __shared__ unsigned s_bal[NR + 2];  // marks of each round
   __shared__ int s_queued;          // marked entries
 
@@ -896,7 +920,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     lp = lf + (k == 0 ? nvr - 1 : k - 1);
     s_lp[t] = lp;
   }
-  if constexpr (PERSIST != 0) {
+  if constexpr (STAGED) {
     if (t == 0) {
       s_far = s_round = s_queued = 0;
     }
@@ -916,7 +940,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     s_seg[t] = seg;
     // ahead of the barrier: the pair phase reads the predecessor's too, and no
     // barrier lies between phase 2 and the unstaged pair phase
-    s_il[t] = rsqrt(fma(seg.y, seg.y, seg.x * seg.x));
+    if constexpr (INTER == INT_SMOOTH) s_il[t] = rsqrt(fma(seg.y, seg.y, seg.x * seg.x));
     const double2 x0 = s_pos[lf];
     const double2 u = pbc2(bx, x, x0);
     const double2 un = pbc2(bx, xn, x0);
@@ -972,7 +996,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
   double esh = 0.0;
   if (t < nvt) {
     // The reference's divisions are taken as products with a few
-    // reciprocals (1/A0, 1/l0 and each segment's 1/l, formed once in phase 1),
+    // reciprocals (1/A0, 1/l0 and the segments' 1/l from one rsqrt each),
     // a rounding-level difference
     const double area = fabs(s_r0[lf]) * 0.5;
     const double inv_a0 = 1.0 / a0r;
@@ -986,7 +1010,14 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     fsh.y += 0.5 * gmA * (npd.x);
     esh += (0.5 * p.ea * dA * dA) / nvr;
     const double ps2 = fma(ps.y, ps.y, ps.x * ps.x), ns2 = fma(ns.y, ns.y, ns.x * ns.x);
-    const double r_pl = s_il[lp], r_nl = s_il[t];  // 1 / |segment|
+    double r_pl, r_nl;  // 1 / |segment|
+    if constexpr (INTER == INT_SMOOTH) {
+      r_pl = s_il[lp];
+      r_nl = s_il[t];
+    } else {
+      r_pl = rsqrt(ps2);
+      r_nl = rsqrt(ns2);
+    }
     const double plen = ps2 * r_pl, nlen = ns2 * r_nl;
     const double tl0 = s_l0[t], pl0 = s_l0[lp];
     if (p.monomer == 0) {
@@ -1021,7 +1052,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
   // L lanes per vertex stride over its list slots; each slot's list entry
   // (neighbour id and packed predecessor offsets) is fetched two slots ahead
   // and the neighbour's three positions one slot ahead, all three together.
-  if constexpr (PERSIST != 0 && INTER == INT_VV) {
+  if constexpr (STAGED && INTER == INT_VV) {
     cp_async_wait_all();
     __syncthreads();
   }
@@ -1034,7 +1065,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
     const GlobalSrc<(PERSIST != 0)> src{pin, a.rad, a.nbr + v0, INTER == INT_SMOOTH ? a.nbr_pq + v0 : nullptr,
                                         (size_t)p.nv, v0};
     bool staged = false;
-    if constexpr (PERSIST != 0) staged = g->on;
+    if constexpr (STAGED) staged = g->on;
     int cnt = 0;
     if (!staged && lv < nvt) cnt = min(__ldg(a.nbr_cnt + v0 + lv), a.nbr_cap);  // an overflowed build stores counts above capacity
     if constexpr (INTER == INT_VV) {
@@ -1065,7 +1096,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
           else pair_own<POT>(p, pbc2(bx, xi, xj), ri + rj, fi, ei);
         }
       };
-      if constexpr (PERSIST != 0) {
+      if constexpr (STAGED) {
         if (staged) pairs(StageSrc<TV>{*g}, g->start[t], g->start[t + 1], 1);
       }
       if (!staged) pairs(src, lane, cnt, L);
@@ -1074,9 +1105,9 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
       // and role 2 (j against i's own segment prev(i) -> i).  The marking pass
       // over the lane's slots (64 at a time) notes in a bit mask those that
       // may contribute, and these run off a queue shared by the warp
-      // (queue_units), in slot order for each vertex: an unmarked slot adds
+      // (queue_lanes), in slot order for each vertex: an unmarked slot adds
       // nothing when evaluated.
-      if constexpr (PERSIST != 0) {
+      if constexpr (STAGED) {
         if (staged) {
           static_assert(L <= 2, "lanes of the staged shapes");
           constexpr int QC = BLOCK / 32 * QN;
@@ -1460,7 +1491,7 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
     return;
   }
   const int4 tile = a.tiles[blockIdx.x];
-  tile_body<POT, INTER, MODE, BLOCK, L, PREC, BATCH, 0>(p, a, s, a.pos, s.pos_out, (unsigned long long)st->rng_step,
+  tile_body<POT, INTER, MODE, BLOCK, L, PREC, BATCH, 0, false>(p, a, s, a.pos, s.pos_out, (unsigned long long)st->rng_step,
                                                         nullptr, false, nullptr, tile);
 }
 
@@ -1547,8 +1578,15 @@ __device__ __forceinline__ int steps_barrier(StepsBarrier& b, bool stop = false)
   return s_ok;
 }
 
-template <int POT, int INTER, int BLOCK, int L, int PREC>
-__global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
+// CTAs an SM the registers are held to: without the stage, five of the
+// vertex-vertex form (740 tiles) rather than four.
+template <int INTER, int BLOCK, int L, int PREC, bool STAGED>
+constexpr int steps_ctas_per_sm() {
+  return INTER == INT_VV && L == 1 && !STAGED ? 5 : tile_threads_per_sm<PREC, L>() / BLOCK;
+}
+
+template <int POT, int INTER, int BLOCK, int L, int PREC, bool STAGED>
+__global__ void __launch_bounds__(BLOCK, (steps_ctas_per_sm<INTER, BLOCK, L, PREC, STAGED>()))
     k_tile_steps(const __grid_constant__ SysParams p, const __grid_constant__ SysArrays a,
                  const __grid_constant__ StepArgs s) {
   pdl_wait();
@@ -1566,13 +1604,13 @@ __global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK)
   extern __shared__ __align__(16) unsigned char s_stage[];
   Stage<BLOCK / L> g(s_stage);
   const int4 tile = a.tiles[blockIdx.x];
-  stage_build<INTER, BLOCK, L>(p, p, a, tile, s.last_pos, s.disp_cutoff, pot_range_f<POT>(p), g);
+  if constexpr (STAGED) stage_build<INTER, BLOCK, L>(p, p, a, tile, s.last_pos, s.disp_cutoff, pot_range_f<POT>(p), g);
   int done = 0;
   bool stalled = false, stopped = false;
   for (int j = 0; j < n; j++) {
     const double2* pin = (j & 1) ? pos1 : pos0;
     double2* pout = (j & 1) ? pos0 : pos1;
-    const bool stop = tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC, false, 1>(
+    const bool stop = tile_body<POT, INTER, MODE_STEP, BLOCK, L, PREC, false, 1, STAGED>(
         p, a, s, pin, pout, step0 + (unsigned long long)j, &st->pflag, j > 0, &g, tile);
     done = j + 1;
     const int b = steps_barrier(bar, stop);

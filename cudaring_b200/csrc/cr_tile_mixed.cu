@@ -37,22 +37,28 @@ void launch_tile_mixed(const LaunchCfg& c, int pot, int inter, int mode, const S
 }
 
 
-// Multi-step kernel (k_tile_steps) for one or two lanes per vertex; nullptr
-// for other lane counts.
+// Multi-step kernel (k_tile_steps): the shapes of tile_steps_fn_fp64.
 template <int POT, int INTER>
-static TileStepsFn steps_fn_l(int lanes) {
-  if (lanes == 1) return k_tile_steps<POT, INTER, 128, 1, PREC_MIXED>;
-  if (lanes == 2) return k_tile_steps<POT, INTER, 192, 2, PREC_MIXED>;
+static TileStepsFn steps_fn_l(int lanes, bool staged) {
+  if (lanes == 1) {
+    if (staged) return k_tile_steps<POT, INTER, 128, 1, PREC_MIXED, true>;
+    return k_tile_steps<POT, INTER, 128, 1, PREC_MIXED, false>;
+  }
+  if (lanes == 2 && staged) return k_tile_steps<POT, INTER, 192, 2, PREC_MIXED, true>;
   return nullptr;
 }
 
-TileStepsFn tile_steps_fn_mixed(int pot, int inter, int lanes) {
-  const bool vv = inter == INT_VV;
+template <int POT>
+static TileStepsFn steps_fn_p(int inter, int lanes, bool staged) {
+  return inter == INT_VV ? steps_fn_l<POT, INT_VV>(lanes, staged) : steps_fn_l<POT, INT_SMOOTH>(lanes, staged);
+}
+
+TileStepsFn tile_steps_fn_mixed(int pot, int inter, int lanes, bool staged) {
   switch (pot) {
-    case POT_HARMONIC: return vv ? steps_fn_l<POT_HARMONIC, INT_VV>(lanes) : steps_fn_l<POT_HARMONIC, INT_SMOOTH>(lanes);
-    case POT_LJ: return vv ? steps_fn_l<POT_LJ, INT_VV>(lanes) : steps_fn_l<POT_LJ, INT_SMOOTH>(lanes);
-    case POT_ADHESIVE: return vv ? steps_fn_l<POT_ADHESIVE, INT_VV>(lanes) : steps_fn_l<POT_ADHESIVE, INT_SMOOTH>(lanes);
-    case POT_WCA: return vv ? steps_fn_l<POT_WCA, INT_VV>(lanes) : steps_fn_l<POT_WCA, INT_SMOOTH>(lanes);
+    case POT_HARMONIC: return steps_fn_p<POT_HARMONIC>(inter, lanes, staged);
+    case POT_LJ: return steps_fn_p<POT_LJ>(inter, lanes, staged);
+    case POT_ADHESIVE: return steps_fn_p<POT_ADHESIVE>(inter, lanes, staged);
+    case POT_WCA: return steps_fn_p<POT_WCA>(inter, lanes, staged);
     default: return nullptr;
   }
 }
