@@ -16,6 +16,7 @@
 // force tolerance, the jammed / under-jammed / over-jammed decision, the
 // saved under-jammed state, and the halving of the compression step when a
 // system overshoots.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,6 +31,7 @@
 #include "cr_tile.cuh"
 
 using namespace cr;
+namespace cg = cooperative_groups;
 
 // Compression protocol state of one system (cr_batch_compress on the device).
 struct CompSys {
@@ -74,6 +76,7 @@ struct cr_batch {
   int ncells = 0, ncells_alloc = 0;
   int4* sgrid = nullptr;  // per system: cells in x, cells in y, first cell, 0
   std::vector<int4> sgrid_h;
+  int cells_cluster = 1;  // CTAs per system of k_bcells
   BatchSys* bsys = nullptr;
   double* bfire = nullptr;  // [S][2][4]
   double* partials = nullptr;
@@ -168,16 +171,23 @@ __device__ __forceinline__ bool b_nothing_due(const BNbr& n) {
   return !st->rebuild || st->abort;
 }
 
-// The cells of a system, by one CTA: counts, starts (the entries of system s
-// are its vertices' own range, its starts begin at its first cell + s, one more
-// than its cells), and its vertices in cell order, ascending ids inside a
-// cell, with the data the search reads.  As count, scan, fill, sort and gather
-// kernels over all systems (the scan by one CTA over every cell of the batch)
-// this took most of a rebuild.
+// The cells of a system, by the CTAs of one cluster (one CTA for systems of a
+// few thousand vertices, cells_cluster): counts, starts (the entries of system
+// s are its vertices' own range, its starts begin at its first cell + s, one
+// more than its cells), and its vertices in cell order, ascending ids inside a
+// cell, with the data the search reads.  The CTAs share the vertices and the
+// runs of cells of the scan; barriers of the cluster in between (no early exit
+// differs between them).
 __global__ void __launch_bounds__(1024) k_bcells(const __grid_constant__ BNbr n) {
   if (b_nothing_due(n)) return;
-  const int s = blockIdx.x, t = threadIdx.x;
-  if (s == 0 && t == 0) {
+  const cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), r = (int)cl.block_rank();
+  const auto sync = [&]() {
+    if (C == 1) __syncthreads();
+    else cl.sync();
+  };
+  const int s = blockIdx.x / C, t = threadIdx.x, first = r * 1024 + t, stride = C * 1024;
+  if (blockIdx.x == 0 && t == 0) {
     n.status->overflow = 0;
     n.status->max_count = 0;
   }
@@ -187,18 +197,19 @@ __global__ void __launch_bounds__(1024) k_bcells(const __grid_constant__ BNbr n)
   const int nc = g.x * g.y, v0 = n.sys_v0[s], v1 = s + 1 < n.S ? n.sys_v0[s + 1] : n.nv;
   int* cnt = n.cell_cnt + g.z;
   int* start = n.cell_start + g.z + s;
-  for (int c = t; c < nc; c += 1024) cnt[c] = 0;
-  __syncthreads();
-  for (int v = v0 + t; v < v1; v += 1024) {
+  for (int c = first; c < nc; c += stride) cnt[c] = 0;
+  sync();
+  for (int v = v0 + first; v < v1; v += stride) {
     const double2 x = n.pos[v];
     const int c = b_cell_coord(x.y, bx.ly, bx.inv_ly, g.y) * g.x + b_cell_coord(x.x, bx.lx, bx.inv_lx, g.x);
     n.cell_of[v] = g.z + c;
     n.slot[v] = atomicAdd(cnt + c, 1);
   }
-  __syncthreads();
-  // exclusive scan, a run of cells per thread
-  __shared__ int s_w[32];
-  const int per = (nc + 1023) / 1024, cb = min(nc, t * per), ce = min(nc, cb + per);
+  sync();
+  // exclusive scan: a part of the cells per CTA, a run of it per thread
+  __shared__ int s_w[32], s_total;
+  const int part = (nc + C - 1) / C, pb = min(nc, r * part), pe = min(nc, pb + part);
+  const int per = (pe - pb + 1023) / 1024, cb = min(pe, pb + t * per), ce = min(pe, cb + per);
   int sum = 0;
   for (int c = cb; c < ce; c++) sum += __ldcg(cnt + c);
   int incl = sum;
@@ -210,17 +221,22 @@ __global__ void __launch_bounds__(1024) k_bcells(const __grid_constant__ BNbr n)
   __syncthreads();
   int run = v0 + incl - sum;
   for (int w = 0; w < (t >> 5); w++) run += s_w[w];
+  if (C > 1) {
+    if (t == 1023) s_total = run - v0 + sum;
+    cl.sync();
+    for (int q = 0; q < r; q++) run += *cl.map_shared_rank(&s_total, q);
+  }
   for (int c = cb; c < ce; c++) {
     start[c] = run;
     run += __ldcg(cnt + c);
   }
-  if (t == 0) start[nc] = v1;
-  __syncthreads();
-  for (int v = v0 + t; v < v1; v += 1024) n.cell_vid[start[n.cell_of[v] - g.z] + n.slot[v]] = v;
-  __syncthreads();
+  if (r == 0 && t == 0) start[nc] = v1;
+  sync();
+  for (int v = v0 + first; v < v1; v += stride) n.cell_vid[start[n.cell_of[v] - g.z] + n.slot[v]] = v;
+  sync();
   // every vertex to its start + the members of its cell with a smaller id; the
   // ids in cell order go to slot, whose per-vertex slots are used up
-  for (int v = v0 + t; v < v1; v += 1024) {
+  for (int v = v0 + first; v < v1; v += stride) {
     const int c = n.cell_of[v] - g.z, b = start[c], e = start[c + 1];
     int rank = 0;
     for (int i = b; i < e; i++) rank += n.cell_vid[i] < v ? 1 : 0;
@@ -724,6 +740,20 @@ double cut_distance_of(const cr_batch* b, double cutoff_) {
   }
 }
 
+// CTAs per system of k_bcells: one for systems of up to 2,048 vertices, else as
+// many as give each SM at most one, up to a cluster of eight.  us with 1, 2, 4
+// and 8 CTAs a system: one of 1,000 vertices 10 / 13 / 13 / 14, 2,000 13.6 / 13.4
+// / 13.2 / 13.4, 10,000 46 / 32 / 23 / 19, 80,000 385 / 196 / 99 / 55, 1.28
+// million 6,480 / 3,270 / 1,630 / 820 (33 us at 20,000, 78 at 80,000 and 1,030 at
+// 1.28 million as count, scan, fill, sort and gather kernels, 23 / 55 / 820 here);
+// 37 systems of 10,000 48 / 32 / 27 / 35, 74 of them 48 / 34 / 46 / 52.
+int cells_cluster(int largest, int systems, int sms) {
+  int c = 1;
+  if (largest > 2048)
+    while (c < 8 && 2 * c * systems <= sms) c *= 2;
+  return c;
+}
+
 // Cell grid of every system for the current boxes, radii and cutDistance.
 int setup_grids(cr_batch* b) {
   b->sgrid_h.assign(b->S, make_int4(1, 1, 0, 0));
@@ -784,7 +814,17 @@ BNbr nbr_args(cr_batch* b, int all) {
 // The batched build as stream-ordered launches (capturable).
 void enqueue_build(cr_batch* b, cudaStream_t st, int all) {
   const BNbr n = nbr_args(b, all);
-  k_bcells<<<b->S, 1024, 0, st>>>(n);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(b->S * b->cells_cluster);
+  cfg.blockDim = dim3(1024);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = b->cells_cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = b->cells_cluster > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_bcells, n);
   k_bnbr<<<(b->nv + 255) / 256, 256, 0, st>>>(n);
   if (all) b->launches += 2;  // builds that only watch a sequence are not counted
 }
@@ -1397,6 +1437,14 @@ int cr_batch_create(long numSystems, const long* numParticles, const long* nvLis
   }
   b->nv = (int)total;
   b->np = (int)rings;
+  {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess) {
+      delete b;
+      return CR_ECUDA;
+    }
+    b->cells_cluster = cells_cluster(*std::max_element(b->sys_nv.begin(), b->sys_nv.end()), b->S, sms);
+  }
   b->bsys_h.assign(b->S, BatchSys{});
   b->box_h.assign(b->S, Box{1.0, 1.0, 1.0, 1.0});
   b->rmax_h.assign(b->S, 0.0);
