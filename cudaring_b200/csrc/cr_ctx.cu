@@ -169,6 +169,8 @@ struct cr_ctx {
   DevStatus* snap_status = nullptr;
 
   std::map<std::tuple<int, long, int, int, unsigned long long>, GraphEntry> graphs;
+  // chunks of each kind run as plain launches since the graphs were last dropped
+  std::map<std::tuple<int, long, int, int, unsigned long long>, int> chunk_uses;
 
   int fail(int code, const std::string& msg) {
     err = msg;
@@ -199,6 +201,7 @@ void drop_graphs(cr_ctx* ctx) {
     if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
   }
   ctx->graphs.clear();
+  ctx->chunk_uses.clear();
   for (auto& kv : ctx->soft_graphs) {
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
@@ -673,20 +676,27 @@ int run_direct(cr_ctx* ctx, const std::vector<Op>& ops, size_t first, int kind) 
   return CR_OK;
 }
 
-// chunks: how many chunks the call runs.  A graph pays once several of them
+// chunks: how many chunks the call runs.  A graph pays once several chunks
 // replay it: capturing, instantiating and destroying one costs some 4 us per op
-// (0.5 ms for 100 rigid steps, whose kernels take 1.5), a plain launch 2 us, less
-// than the op takes.
-constexpr size_t kGraphChunks = 8;
+// (0.5 ms for 100 rigid steps, whose kernels take 1.5), a replay saves 0.4 to 3 us
+// a step over plain launches (us per step, plain / replayed: 16 rigid rings 8.6
+// / 8.1, 4,096 of them 18.0 / 17.3; NVERescale of 4,800 vertices 16.1 / 13.3, of
+// 98,304 32.8 / 29.7).  So the first chunks of a kind go out as plain launches,
+// and from the eighth on, in one call or over several, they replay a graph.
+constexpr int kGraphChunks = 8;
+constexpr size_t kChunkKinds = 256;
 int launch_chunk(cr_ctx* ctx, const std::vector<Op>& ops, int kind, long n, size_t chunks) {
-  if (ctx->use_graphs && chunks < kGraphChunks) {
-    const long long before = ctx->launches;
-    ctx->launches = before + enqueue_chunk(ctx, ops, kind);
-    CR_TRY(cudaGetLastError());
-    return CR_OK;
+  const auto key = std::make_tuple(kind, n, ops.front().in_buf, ctx->cap, 0ULL);
+  if (ctx->use_graphs && chunks < (size_t)kGraphChunks && !ctx->graphs.count(key)) {
+    if (ctx->chunk_uses.size() >= kChunkKinds) ctx->chunk_uses.clear();
+    if (++ctx->chunk_uses[key] < kGraphChunks) {
+      const long long before = ctx->launches;
+      ctx->launches = before + enqueue_chunk(ctx, ops, kind);
+      CR_TRY(cudaGetLastError());
+      return CR_OK;
+    }
   }
   if (ctx->use_graphs) {
-    auto key = std::make_tuple(kind, n, ops.front().in_buf, ctx->cap, 0ULL);
     auto it = ctx->graphs.find(key);
     if (it == ctx->graphs.end()) {
       GraphEntry ge;
