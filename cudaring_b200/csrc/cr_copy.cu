@@ -68,8 +68,24 @@ cudaError_t plain(cudaStream_t st, void* dst, const void* src, size_t bytes, boo
   return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 }
 
+// The context's device for one copy, the caller's again after it: a plain copy
+// runs on a stream of any device, but events belong to the device that was
+// current when they were made.
+struct OnDevice {
+  int before = -1;
+  explicit OnDevice(int device) {
+    int now;
+    if (cudaGetDevice(&now) != cudaSuccess || now == device) return;
+    if (cudaSetDevice(device) == cudaSuccess) before = now;
+  }
+  ~OnDevice() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
 cudaError_t copy(Staging& s, int device, cudaStream_t st, void* dst, const void* src, size_t bytes, bool in) {
   if (bytes < kLarge) return plain(st, dst, src, bytes, in);
+  const OnDevice on(device);
   cudaPointerAttributes at{};
   const cudaError_t e = cudaPointerGetAttributes(&at, in ? src : dst);
   if (e != cudaSuccess) cudaGetLastError();
