@@ -26,18 +26,26 @@
 namespace cr {
 
 
-// Occupancy target in threads per SM.  One lane per vertex: 512 leaves 128
-// registers per thread, where the FP64 smooth-interaction body compiles
-// without spills.  Two lanes per vertex (192-thread CTAs, tiles of up to 96
-// vertices): 576 threads (three CTAs, 96 registers), so that the grid of a
-// 39,424-vertex system (about 430 tiles) runs as one wave.  The mixed path
-// takes the same budgets: it holds an FP64 unit body for its near-contact
-// slots beside the FP32 one, and at 80 registers (four CTAs) its spills cost
-// more than the fourth CTA gains (27.5 against 25.5 us per step measured at
-// 39,424 vertices).
+// Occupancy target in threads per SM, smooth interaction.  One lane per vertex:
+// 512 leaves 128 registers per thread.  Two lanes per vertex (192-thread CTAs,
+// tiles of up to 96 vertices): 576 threads (three CTAs, 96 registers), so that
+// the grid of a 39,424-vertex system (about 430 tiles) runs as one wave.  The
+// FP64 body spills 44 to 148 bytes in one op per launch and 120 to 360 with the
+// staged queue of the multi-step kernels.  The mixed path takes the same
+// budgets: it holds an FP64 unit body for its near-contact slots beside the
+// FP32 one, and at 80 registers (four CTAs) its spills cost more than the fourth
+// CTA gains (27.5 against 25.5 us per step measured at 39,424 vertices).
 template <int PREC, int L = 1>
 constexpr int tile_threads_per_sm() {
   return L >= 2 ? 576 : 512;
+}
+// One op per launch with vertex-vertex pairs: 768 threads (80 registers) hold
+// four CTAs of 192, three of 256 or six of 128.  Left to itself the compiler
+// takes 82 to 88 and an SM holds one CTA less (four lanes, us per step: 1,500
+// rings of 24 vertices 16.8 -> 13.0, 4,096 rings 34.3 -> 26.3).
+template <int INTER, int BLOCK, int PREC, int L>
+constexpr int tile_ctas_per_sm() {
+  return (INTER == INT_VV ? 768 : tile_threads_per_sm<PREC, L>()) / BLOCK;
 }
 
 template <typename T2> __device__ __forceinline__ T2 cvt2(double2 d);
@@ -1471,7 +1479,7 @@ __device__ __forceinline__ bool tile_body(const SysParams& p, const SysArrays& a
 }
 
 template <int POT, int INTER, int MODE, int BLOCK, int L, int PREC, bool BATCH = false>
-__global__ void __launch_bounds__(BLOCK, tile_threads_per_sm<PREC, L>() / BLOCK) k_tile(const __grid_constant__ SysParams p,
+__global__ void __launch_bounds__(BLOCK, (tile_ctas_per_sm<INTER, BLOCK, PREC, L>())) k_tile(const __grid_constant__ SysParams p,
                                                 const __grid_constant__ SysArrays a,
                                                 const __grid_constant__ StepArgs s) {
   // every input may come from the kernel before this one (positions, lists,
