@@ -528,7 +528,7 @@ __device__ __forceinline__ void reduce_partials(const double* partials, int nblo
   }
 }
 
-// Sums of N arrays over v[f .. f + n) (stride `st` doubles, n <= 256) by one
+// Sums of N arrays over v[f .. f + n) (n <= 256) by one
 // warp, left in v[f], as a tree of neighbours: ((0 + 1) + (2 + 3)) + ..., each
 // lane its own run of 1, 2, 4 or 8 elements first.  The order is that of a tree
 // over shared memory with strides 1, 2, 4, ..: the stiff area term multiplies
@@ -537,15 +537,15 @@ __device__ __forceinline__ void reduce_partials(const double* partials, int nblo
 // striding over the ring, 200 steps of the 39,424-vertex mixed run ended 1e-9
 // away).
 template <int N>
-__device__ __forceinline__ void ring_sums(double* const (&v)[N], int f, int n, int st = 1) {
+__device__ __forceinline__ void ring_sums(double* const (&v)[N], int f, int n) {
   const int wl = threadIdx.x & 31;
   const int run = n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : 8;
   const int c = wl * run;
   double x[N];
 #pragma unroll
   for (int q = 0; q < N; q++) {
-    const double* e = v[q] + (size_t)f * st;
-    const auto at = [&](int k) { return k < n ? e[k * st] : 0.0; };
+    const double* e = v[q] + f;
+    const auto at = [&](int k) { return k < n ? e[k] : 0.0; };
     if (run == 1) x[q] = at(c);
     else if (run == 2) x[q] = at(c) + at(c + 1);
     else {
@@ -553,12 +553,26 @@ __device__ __forceinline__ void ring_sums(double* const (&v)[N], int f, int n, i
       if (run == 8) x[q] += (at(c + 4) + at(c + 5)) + (at(c + 6) + at(c + 7));
     }
   }
-  for (int o = 1; o < 32; o <<= 1)
+  if constexpr (N == 4) {
+    // the lanes share the arrays out while they add: after the first exchange a
+    // lane holds two of them, after the second one (6 exchanges of a double in
+    // place of 20; the same sums)
+    const bool b0 = wl & 1, b1 = wl & 2;
+    double y = b0 ? x[2] : x[0], z = b0 ? x[3] : x[1];
+    y += __shfl_xor_sync(0xffffffffu, b0 ? x[0] : x[2], 1);
+    z += __shfl_xor_sync(0xffffffffu, b0 ? x[1] : x[3], 1);
+    double w = b1 ? z : y;
+    w += __shfl_xor_sync(0xffffffffu, b1 ? y : z, 2);
+    for (int o = 4; o < 32; o <<= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if (wl < 4) (b0 ? (b1 ? v[3] : v[2]) : (b1 ? v[1] : v[0]))[f] = w;
+  } else {
+    for (int o = 1; o < 32; o <<= 1)
 #pragma unroll
-    for (int q = 0; q < N; q++) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
-  if (wl == 0)
+      for (int q = 0; q < N; q++) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
+    if (wl == 0)
 #pragma unroll
-    for (int q = 0; q < N; q++) v[q][(size_t)f * st] = x[q];
+      for (int q = 0; q < N; q++) v[q][f] = x[q];
+  }
 }
 
 }  // namespace cr
