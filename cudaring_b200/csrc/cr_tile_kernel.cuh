@@ -716,6 +716,7 @@ __device__ __forceinline__ void queue_lanes(const SysParams& p, const B& bx, con
   constexpr unsigned kAll = 0xffffffffu;
   const int wl = threadIdx.x & 31;
   const int n = __popcll(need);
+  if (!__any_sync(kAll, n != 0)) return;
   int incl = n;
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(kAll, incl, o);
