@@ -1,6 +1,6 @@
 // Context, op sequencer (step ops, each followed by the one-launch neighbour
-// build that runs only when the op armed it, launched one by one or, in calls
-// of many chunks, as a captured graph; sequences of steps and of FIRE
+// build that runs only when the op armed it, launched one by one or, once a
+// chunk has run a few times, as a captured graph; sequences of steps and of FIRE
 // iterations in multi-step kernels) and the C ABI declared in
 // include/cudaring.h.
 #include <algorithm>
@@ -951,9 +951,10 @@ int run_fire_steps(cr_ctx* ctx, FireStepsFn fn, long nsteps) {
   return CR_OK;
 }
 
-// Runs nsteps integrator steps (or FIRE iterations) as chunks of captured
-// graphs.  Non-FIRE chunks are launched back to back with one status read at
-// the end; FIRE reads the status after every chunk to stop at convergence.
+// Runs nsteps integrator steps (or FIRE iterations): in multi-step launches where
+// these serve the run, else in chunks of up to 128 (launch_chunk).  Non-FIRE
+// chunks are launched back to back with one status read at the end; FIRE reads
+// the status after every chunk to stop at convergence.
 // A neighbour-list overflow inside a chunk aborts the remaining ops (they
 // become no-ops); the host then grows the list and resumes from the op after
 // which the failed build ran.

@@ -324,17 +324,19 @@ int cr_profile_step_kernel(cr_ctx* ctx, long reps, double* ms_per_launch);
 int cr_set_lanes(cr_ctx* ctx, int lanes);
 int cr_get_lanes(const cr_ctx* ctx, int* lanes);
 /* 1 (default): step sequences go to the stream without host checks between
- * ops (as a captured CUDA graph where a call replays it at least eight times,
- * else as plain launches, or in a multi-step kernel), every op that moved
- * positions followed by the one-launch rebuild check; 0: direct launches with
- * a host check after each op. */
+ * ops (in a multi-step kernel, or in chunks of up to 128 steps: plain launches
+ * at first, a captured CUDA graph from a chunk's eighth run on), every op that
+ * moved positions followed by the one-launch rebuild check; 0: direct launches
+ * with a host check after each op. */
 int cr_set_use_graphs(cr_ctx* ctx, int on);
 /* 1 (default): the middle steps of NVE, Langevin and BAOAB runs of
  * deformable rings, and their FIRE iterations in FP64, run in a multi-step
  * kernel (up to 64 steps per launch, grid barriers between steps) when the
- * GPU holds all of its CTAs at once and one or two lanes per vertex are in
- * use; 0: one launch per op.  FP64
- * step results are identical, FIRE's agree to rounding; mixed-precision results agree to FP32 rounding.
+ * GPU holds all of its CTAs (one per tile) at once and one or two lanes per
+ * vertex are in use: on a B200 444 tiles with two lanes; with one lane 740
+ * (steps, vertex-vertex), 592 (steps, smooth; FIRE, vertex-vertex) or 296
+ * (FIRE, smooth); 0: one launch per op.  FP64 step results are identical,
+ * FIRE's agree to rounding; mixed-precision results agree to FP32 rounding.
  * The kernel's grid barriers need all of its CTAs resident (so does the
  * one-launch neighbour-list build).  With other work running on the same
  * GPU a barrier may give up (cr_set_spin_limit); the context then goes back
