@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <string>
 #include <vector>
@@ -1001,18 +1002,23 @@ int add_fire_iterations(cr_batch* b, cudaStream_t st, long n) {
 // 32 systems of 1,200 vertices 29.4 / 19.7, four lanes 39.7 / 25.7; 96 of 2,000
 // 46.8 / 34.9, smooth, two lanes 79.8 / 72.3).
 int run_fire_chunk(cr_batch* b, long n, long whole) {
-  int rc;
   if (n == whole && !b->fire_chunk && ++b->fire_chunks >= 4) {
     const long long launches = b->launches;
     cudaGraph_t graph = nullptr;
-    BT_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    rc = add_fire_iterations(b, b->stream, n);
+    cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      const int rc = add_fire_iterations(b, b->stream, n);
+      e = cudaStreamEndCapture(b->stream, &graph);
+      if (!rc && e == cudaSuccess && cudaGraphInstantiate(&b->fire_chunk, graph, 0) != cudaSuccess)
+        b->fire_chunk = nullptr;
+    }
     b->launches = launches;
-    cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
-    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&b->fire_chunk, graph, 0);
     if (graph) cudaGraphDestroy(graph);
-    if (rc) return rc;
-    BT_TRY(e);
+    if (!b->fire_chunk) {
+      // no graph to be had: plain launches until the next initialisation
+      cudaGetLastError();
+      b->fire_chunks = std::numeric_limits<int>::min();
+    }
   }
   if (n == whole && b->fire_chunk) {
     BT_TRY(cudaGraphLaunch(b->fire_chunk, b->stream));
